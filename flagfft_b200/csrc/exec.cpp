@@ -33,6 +33,7 @@
 
 #include "batch.cuh"
 #include "exec_internal.hpp"
+#include "mixed.cuh"
 #include "tables.hpp"
 
 namespace ffb {
@@ -416,6 +417,7 @@ static Core make_dit_core(int64_t L, const std::vector<int> &r) {
     c.span[s] = (int)span;
     c.sdiv[s] = make_fastdiv((uint32_t)span);
     c.rdiv[s] = make_fastdiv((uint32_t)r[s]);
+    c.bdiv[s] = make_fastdiv((uint32_t)(L / r[s]));
     span *= r[s];
   }
   if (span != L) throw std::runtime_error("radices do not multiply to the core length");
@@ -433,6 +435,7 @@ static Core make_dif_core(int64_t L, const std::vector<int> &r) {
     c.span[s] = (int)span;
     c.sdiv[s] = make_fastdiv((uint32_t)(span / r[s]));
     c.rdiv[s] = make_fastdiv((uint32_t)r[s]);
+    c.bdiv[s] = make_fastdiv((uint32_t)(L / r[s]));
     span /= r[s];
   }
   if (span != 1) throw std::runtime_error("radices do not multiply to the core length");
@@ -552,6 +555,118 @@ class Builder {
     return pow2 ? tpt : choose_tpt(L, {rmin});
   }
 
+  static bool W_overflows(int64_t W, int64_t L, long long g, long long i) {
+    return W * std::llabs(g) + L * std::llabs(i) >= (1ll << 31);
+  }
+
+  // Radix chain of the pass on the mixed-radix tile kernel (mixed.cuh), or
+  // empty when another kernel takes it: a compile-time row, tile or TMA
+  // column sequence, a pass of a batch program (whose persistent kernel runs
+  // the ping-pong body), a single codelet, a layout the kernel does not read,
+  // or two buffers too long for one CTA.  The first and last stage move runs
+  // of L/R0 and L/R_last elements of global memory, so both are kept at four
+  // (32 bytes in single precision) or more.
+  static std::vector<int> mixed_radices(const CoreSpec &spec, IoKind io, int64_t nbatch, int64_t G, long long ib,
+                                        long long ig, long long ii, long long ob, long long og, long long ok) {
+    const int64_t L = spec.L;
+    std::vector<int> seq, sorted_r = spec.radices;
+    std::sort(sorted_r.rbegin(), sorted_r.rend());
+    if (t_no_one_pass || L < 2) return {};
+    const bool fixed = fixed_sequence(L, &seq) && seq == sorted_r;
+    const bool strided = ii > ig || ok > og;
+    if (io == IoKind::C2C) {
+      if (spec.kind == CoreKind::Dit && spec.radices.size() == 1) return {};
+      if (fixed && spec.kind != CoreKind::Rader && ii == 1 && ok == 1) return {};
+      if (fixed && spec.kind == CoreKind::Dit && strided) {
+        int tw = 0, th = 0;
+        size_t sm = 0;
+        if (tiles_shape<T>((int)L, &tw, &th, &sm)) return {};
+        if (tma_columns_enabled() && tcols_eligible<T>((int)L, nbatch, G, ib, ig, ii, ob, og, ok, &th, &sm)) return {};
+      }
+    } else if (io == IoKind::R2C ? (ii != 2 || ok != 1) : io == IoKind::C2R ? (ii != 1 || ok != 2)
+               : io == IoKind::R2CFull || io == IoKind::C2RFull ? (ii != 1 || ok != 1) : true) {
+      return {};
+    }
+    if (nbatch > 65535) return {};
+    std::vector<int> r;
+    if (!mixed_chain(L, 0, &r) && !mixed_chain(L, 1, &r)) return {};
+    if (r.size() < 2 || (int)r.size() > kMaxStages || L / r.front() < 4 || L / r.back() < 4) return {};
+    Core c{};
+    c.L = (int)L;
+    c.nst = (int)r.size();
+    c.radix[0] = r[0];
+    const size_t per = ((size_t)mixed::slot_len(c, mixed::buffers(c, spec.kind, io)) + 2) * sizeof(cpx<T>);
+    return per <= 232448 ? r : std::vector<int>{};
+  }
+
+  // Cheapest chain of the radix set (stage_cost per element), largest first;
+  // false when the length has none.
+  static bool mixed_chain(int64_t L, int set, std::vector<int> *out) {
+    std::map<int64_t, std::pair<double, int>> memo;
+    std::function<double(int64_t)> best = [&](int64_t m) -> double {
+      if (m == 1) return 0.0;
+      auto it = memo.find(m);
+      if (it != memo.end()) return it->second.first;
+      std::pair<double, int> b{1e30, 0};
+      for (int64_t R : kSupportedRadices) {
+        if (m % R || !mixed::in_set<T>(set, (int)R)) continue;
+        const double c = stage_cost((int)R) + best(m / R);
+        if (c < b.first) b = {c, (int)R};
+      }
+      memo[m] = b;
+      return b.first;
+    };
+    if (best(L) > 1e29) return false;
+    out->clear();
+    for (int64_t v = L; v > 1; v /= memo.at(v).second) out->push_back(memo.at(v).second);
+    std::sort(out->rbegin(), out->rend());
+    return true;
+  }
+
+  // Transforms per tile (a.W) and threads per CTA (a.mixed) of a mixed-radix
+  // pass; returns its shared memory.  The shape with the least modelled time
+  // is taken: per SM, the waves of resident tiles, each the longer of the
+  // issue time of the tiles' butterflies (rounds of whole CTAs, so a shape
+  // whose stages leave threads without a butterfly costs more) and one tile's
+  // own latency (its rounds in sequence, a barrier per stage, two global
+  // round trips).
+  static size_t choose_mixed(TileArgs<T> &a, CoreKind kind, IoKind io, bool strided) {
+    const int regs = sizeof(T) == 4 ? (a.mixed_set == 0 ? 80 : 128) : (a.mixed_set == 0 ? 128 : 255);
+    const int64_t most = std::min<int64_t>(a.G, 64);
+    int64_t least = 1;
+    if (strided)
+      for (least = std::min<int64_t>(sizeof(T) == 4 ? 8 : 4, a.G);
+           least > 1 && mixed::smem_bytes(a, kind, io, (int)least) > 232448; --least) {
+      }
+    double best = 1e300;
+    for (int NT = 64; NT <= mixed::kMaxThreads; NT += 32)
+      for (int64_t W = least; W <= most; ++W) {
+        const size_t smem = mixed::smem_bytes(a, kind, io, (int)W);
+        if (smem > 232448) break;
+        const int64_t per_sm = std::min<int64_t>({65536 / (regs * NT), (int64_t)(232448 / (smem + 1024)), 2048 / NT, 32});
+        if (per_sm < 1) continue;
+        const int64_t tiles = a.nbatch * ((a.G + W - 1) / W);
+        double issue = 0, latency = 2000;
+        for (const Core *c : {&a.core, &a.core2})
+          for (int s = 0; s < c->nst; ++s) {
+            const double rounds = (double)((W * (c->L / c->radix[s]) + NT - 1) / NT);
+            const double instr = stage_cost(c->radix[s]) * c->radix[s];
+            issue += rounds * instr * (NT / 32) / 4;
+            latency += rounds * instr * 3 + 100;
+          }
+        const double waves = (double)((tiles + kSMs * per_sm - 1) / (kSMs * per_sm));
+        const double resident = (double)std::min<int64_t>(per_sm, (tiles + kSMs - 1) / kSMs);
+        const double time = waves * std::max(resident * issue, latency);
+        if (time < best * 0.999) {
+          best = time;
+          a.W = (int)W;
+          a.mixed = NT;
+        }
+      }
+    if (!a.mixed) throw std::runtime_error("no tile shape for a mixed-radix pass");
+    return mixed::smem_bytes(a, kind, io, a.W);
+  }
+
   // Fill a tile pass for G transforms per outer batch.
   TilePass<T> *add_pass(const CoreSpec &spec, IoKind io, bool inverse, int64_t nbatch, int64_t G, long long ib,
                         long long ig, long long ii, long long ob, long long og, long long ok, Buf src, Buf dst,
@@ -579,15 +694,17 @@ class Builder {
     std::vector<int> seq, sorted_r = spec.radices;
     std::sort(sorted_r.rbegin(), sorted_r.rend());
     const size_t rows_per = ((size_t)pp_size((int)L) + 1) * sizeof(cpx<T>);
+    const std::vector<int> mixed_r = mixed_radices(spec, io, nbatch, G, ib, ig, ii, ob, og, ok);
     const bool rows_only = io == IoKind::C2C && L > 1 && pp_per > limit && rows_per <= limit && ii == 1 &&
                            ok == 1 && ii <= ig && fixed_sequence(L, &seq) && seq == sorted_r;
     a.pp = (io == IoKind::C2C && L > 1 && (pp_per <= limit || rows_only)) ? 1 : 0;
     a.rows_only = (a.pp && pp_per > limit) ? 1 : 0;
+    if (!mixed_r.empty()) a.pp = 1;
     // ping-pong cores run their radices largest first (any order is the same
     // DFT; this one matches the compile-time sequences), and a convolution's
     // inverse core the same order; the in-place pair needs DIF then DIT with
     // the radices reversed
-    std::vector<int> radices = spec.radices;
+    std::vector<int> radices = mixed_r.empty() ? spec.radices : mixed_r;
     if (a.pp) std::sort(radices.rbegin(), radices.rend());
     if (spec.kind == CoreKind::Dit) {
       a.core = make_dit_core(L, radices);
@@ -620,6 +737,24 @@ class Builder {
       // convolution: forward core (DIF in place, DIT for Stockham), inverse core2
       a.tw = table_stage_twiddles(a.core, a.pp == 0, false);
       a.tw2 = table_stage_twiddles(a.core2, false, true);
+    }
+    if (!mixed_r.empty()) {
+      a.wfast = ii > ig ? 1 : 0;
+      for (int r : mixed_r)
+        if (!mixed::in_set<T>(0, r)) a.mixed_set = 1;
+      p->smem = choose_mixed(a, spec.kind, io, ii > ig || ok > og);
+      if (W_overflows(a.W, L, ig, ii) || W_overflows(a.W, L, og, ok))
+        throw std::runtime_error("tile extent above 2^31 elements");
+      a.tpt = 1;
+      a.wdiv = make_fastdiv((uint32_t)a.W);
+      a.pairs_div = make_fastdiv((uint32_t)(std::max<int64_t>(0, logical_n) / 2 / 2 + 1));
+      p->kind = spec.kind;
+      p->io = io;
+      p->src = src;
+      p->dst = dst;
+      TilePass<T> *raw = p.get();
+      prog_.passes.push_back(std::move(p));
+      return raw;
     }
     // thread and tile shape: column tiles (transform index fastest in memory)
     // take consecutive transforms on consecutive threads
@@ -678,7 +813,7 @@ class Builder {
       }
     }
     // offsets inside one CTA's tile are 32-bit in the kernels
-    if (W * std::llabs(ig) + L * std::llabs(ii) >= (1ll << 31) || W * std::llabs(og) + L * std::llabs(ok) >= (1ll << 31))
+    if (W_overflows(W, L, ig, ii) || W_overflows(W, L, og, ok))
       throw std::runtime_error("tile extent above 2^31 elements");
     const size_t smem = a.tiles ? smem_tiles : per * (size_t)W;
     a.ldiv = make_fastdiv((uint32_t)L);

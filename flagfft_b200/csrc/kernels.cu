@@ -9,23 +9,36 @@
 
 namespace ffb {
 
-namespace tile {
-// defined in k_*.cu
-template <typename T, int K>
-cudaError_t launch_group(const TileArgs<T> &a, int io, size_t smem, cudaStream_t s);
-template <typename T, int K, bool INV>
-cudaError_t launch_pp(const TileArgs<T> &a, size_t smem, cudaStream_t s);
-template <typename T, int KIND, bool INV>
-cudaError_t launch_pp_fixed_any(const TileArgs<T> &a, size_t smem, cudaStream_t s);
-template <typename T, int KIND, int IO>
-cudaError_t launch_one(const TileArgs<T> &a, size_t smem, cudaStream_t s);
-}  // namespace tile
+// (declared extern so that this file does not compile every kernel again)
+#define FFB_EXTERN(T)                                                                                       \
+  namespace rows {                                                                                          \
+  extern template cudaError_t launch_rows_any<T, 0, false>(const TileArgs<T> &, size_t, cudaStream_t);      \
+  extern template cudaError_t launch_rows_any<T, 0, true>(const TileArgs<T> &, size_t, cudaStream_t);       \
+  extern template cudaError_t launch_rows_any<T, 1, false>(const TileArgs<T> &, size_t, cudaStream_t);      \
+  extern template cudaError_t launch_rows_any<T, 3, false>(const TileArgs<T> &, size_t, cudaStream_t);      \
+  }                                                                                                         \
+  namespace tile {                                                                                          \
+  extern template cudaError_t launch_group<T, 0>(const TileArgs<T> &, int, size_t, cudaStream_t);           \
+  extern template cudaError_t launch_group<T, 1>(const TileArgs<T> &, int, size_t, cudaStream_t);           \
+  extern template cudaError_t launch_group<T, 2>(const TileArgs<T> &, int, size_t, cudaStream_t);           \
+  extern template cudaError_t launch_one<T, 0, 5>(const TileArgs<T> &, size_t, cudaStream_t);               \
+  extern template cudaError_t launch_one<T, 0, 6>(const TileArgs<T> &, size_t, cudaStream_t);               \
+  extern template cudaError_t launch_one<T, 3, 0>(const TileArgs<T> &, size_t, cudaStream_t);               \
+  extern template cudaError_t launch_pp<T, 0, false>(const TileArgs<T> &, size_t, cudaStream_t);            \
+  extern template cudaError_t launch_pp<T, 0, true>(const TileArgs<T> &, size_t, cudaStream_t);             \
+  extern template cudaError_t launch_pp<T, 1, false>(const TileArgs<T> &, size_t, cudaStream_t);            \
+  extern template cudaError_t launch_pp<T, 2, false>(const TileArgs<T> &, size_t, cudaStream_t);            \
+  extern template cudaError_t launch_pp<T, 3, false>(const TileArgs<T> &, size_t, cudaStream_t);            \
+  }
+FFB_EXTERN(float)
+FFB_EXTERN(double)
+#undef FFB_EXTERN
 
-namespace rows {
-// defined in k_*_rows*.cu
-template <typename T, int KIND, bool INV>
-cudaError_t launch_rows_any(const TileArgs<T> &a, size_t smem, cudaStream_t s);
-}  // namespace rows
+namespace mixed {
+// defined in k_*_mixed*.cu
+template <typename T, int K>
+cudaError_t launch(const TileArgs<T> &a, IoKind io, size_t smem, cudaStream_t s);
+}  // namespace mixed
 
 namespace {
 
@@ -376,9 +389,18 @@ cudaError_t launch_tile(const TileArgs<T> &a, CoreKind kind, IoKind io, size_t s
     if (e != cudaErrorNotSupported) return e;  // else: buffers off the copy rules, the tile kernels below
   }
   if (a.tiles) return launch_tiles<T>(a, s);
+  if (a.mixed) {
+    switch (k) {
+      case 0: return mixed::launch<T, 0>(a, io, smem, s);
+      case 1: return mixed::launch<T, 1>(a, io, smem, s);
+      case 2: return mixed::launch<T, 2>(a, io, smem, s);
+      case 3: return mixed::launch<T, 3>(a, io, smem, s);
+      default: return cudaErrorInvalidValue;
+    }
+  }
   if (a.pp && o == 0) {
-    // compile-time radix sequences first: contiguous rows, then any layout
-    // (cudaErrorNotSupported: no kernel for this pass)
+    // contiguous rows of a compile-time radix sequence first
+    // (cudaErrorNotSupported: no row kernel for this pass)
     if (k == 0 || k == 1 || k == 3) {
       const cudaError_t e = k == 0 ? (a.inv ? rows::launch_rows_any<T, 0, true>(a, smem, s)
                                             : rows::launch_rows_any<T, 0, false>(a, smem, s))
@@ -387,13 +409,6 @@ cudaError_t launch_tile(const TileArgs<T> &a, CoreKind kind, IoKind io, size_t s
       if (e != cudaErrorNotSupported) return e;
     }
     if (a.rows_only) return cudaErrorInvalidConfiguration;  // no general tile fits its shared memory
-    if (k == 0 || k == 1 || k == 3) {
-      const cudaError_t e = k == 0 ? (a.inv ? tile::launch_pp_fixed_any<T, 0, true>(a, smem, s)
-                                            : tile::launch_pp_fixed_any<T, 0, false>(a, smem, s))
-                            : k == 1 ? tile::launch_pp_fixed_any<T, 1, false>(a, smem, s)
-                                     : tile::launch_pp_fixed_any<T, 3, false>(a, smem, s);
-      if (e != cudaErrorNotSupported) return e;
-    }
     switch (k) {
       case 0: return a.inv ? tile::launch_pp<T, 0, true>(a, smem, s) : tile::launch_pp<T, 0, false>(a, smem, s);
       case 1: return tile::launch_pp<T, 1, false>(a, smem, s);
@@ -415,7 +430,7 @@ size_t tile_smem(const TileArgs<T> &a, CoreKind kind, IoKind io, size_t smem) {
   const int k = (int)kind;
   if (a.regcol) return 0;
   if (a.blue_cols) return blue4_smem(a.blue_cols, a.core.L, sizeof(cpx<T>), a.blue_pair != 0);
-  if (a.tiles) return smem;
+  if (a.tiles || a.mixed) return smem;
   if (a.pp && io == IoKind::C2C && (k == 0 || k == 1 || k == 3)) {
     const size_t r = k == 0 ? rows::rows_smem_any<T, 0>(a) : k == 1 ? rows::rows_smem_any<T, 1>(a)
                                                                      : rows::rows_smem_any<T, 3>(a);

@@ -138,6 +138,14 @@ struct TileArgs {
   int tcols;
   int tc_threads;
   int tc_smem;
+  // > 0: the pass runs on the mixed-radix tile kernel (mixed.cuh) with this
+  // many threads per CTA and its radix set (the ping-pong configuration's convolution tables:
+  // natural order).  pairs_div divides by n/4 + 1 (half-length real
+  // transforms); pair_aligned is set at launch.
+  int mixed;
+  int mixed_set;
+  int pair_aligned;
+  FastDiv pairs_div;
 };
 
 // Shared memory the general ping-pong tile body needs for a pass's W
