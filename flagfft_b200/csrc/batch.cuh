@@ -1,19 +1,24 @@
 // Persistent batch kernel: one launch runs a queue of work items drawn from
 // many plans of different lengths (the passes of one phase of a batch
 // program).  Each CTA takes the next item from a device counter, runs it with
-// the same tile bodies as the per-plan kernels, and loops until the queue is
+// the mixed-radix tile body (mixed.cuh) or the in-place one, and loops until the queue is
 // empty, so lengths of very different cost share the GPU without a launch per
 // length.  An item is (index of its pass's TileArgs, tile index):
 //   ping-pong passes (kinds 0-3 = Dit, Bluestein, Rader, Conv): tile =
 //     by * ceil(G / W) + bx, the CTA tile of the per-plan launch;
 //   register-column passes (kind 8): tile = by * ceil(G / blockDim) + chunk,
 //     blockDim consecutive transforms, one per thread.
-// The CTA is as wide as the widest item of the launch; a narrower ping-pong
-// item leaves the extra threads idle through its stages (they still meet
-// every barrier).
+// The CTA is as wide as the widest item of the launch.  A ping-pong item's
+// butterflies are spread over all its threads; a narrower in-place item
+// leaves the extra threads idle through its stages (they still meet every
+// barrier).  With the mixed-radix body instead of the ping-pong one, which kept
+// W * tpt threads and a load and a store phase, 600 transforms of 16 to 16384
+// points went from 131.7 to 113.2 us on one B200 (what bounds them: the longest
+// convolutions, one CTA each).
 #pragma once
 
 #include "kernels.cuh"
+#include "mixed.cuh"
 #include "regcol.cuh"
 #include "tile_impl.cuh"
 
@@ -28,6 +33,12 @@ enum BatchKind : int {
   kBatchC2R = 5,  // the same with the Hermitian pre / unpack
   kBatchRegcol = 8
 };
+
+// Shared memory of a ping-pong pass's items at its tile width.
+template <typename T>
+inline size_t batch_item_smem(const TileArgs<T> &a, CoreKind kind) {
+  return mixed::smem_bytes(a, kind, IoKind::C2C, a.W);
+}
 
 struct BatchItem {
   int args;
@@ -111,15 +122,15 @@ FFB_HD void run_item(const TileArgs<T> &a, int kind, int tile, cpx<T> *sm, const
     tile::tile_body<T, 0, (int)IoKind::C2R>(a, bx, by, sm, x);
   } else if (kind == kBatchPpDit) {
     if (a.inv)
-      tile::tile_body_pp<T, 0, true>(a, bx, by, sm, x);
+      mixed::body<T, 0, false, true, 1, true>(a, 0, bx, by, sm, x);
     else
-      tile::tile_body_pp<T, 0, false>(a, bx, by, sm, x);
+      mixed::body<T, 0, false, false, 1, true>(a, 0, bx, by, sm, x);
   } else if (kind == kBatchPpBluestein) {
-    tile::tile_body_pp<T, 1, false>(a, bx, by, sm, x);
+    mixed::body<T, 1, false, false, 1>(a, 0, bx, by, sm, x);
   } else if (kind == kBatchPpRader) {
-    tile::tile_body_pp<T, 2, false>(a, bx, by, sm, x);
+    mixed::body<T, 2, false, false, 1>(a, 0, bx, by, sm, x);
   } else {
-    tile::tile_body_pp<T, 3, false>(a, bx, by, sm, x);
+    mixed::body<T, 3, false, false, 1>(a, 0, bx, by, sm, x);
   }
 }
 

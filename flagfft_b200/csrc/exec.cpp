@@ -1915,7 +1915,7 @@ std::unique_ptr<BatchProgram> lower_batch_t(const std::vector<BatchGroup> &group
           tp->a.tpt > kBatchWidth)
         continue;
       TileArgs<T> &a = tp->a;
-      const size_t per = pp_tile_smem(a) / (size_t)a.W;
+      const size_t per = batch_item_smem(a, tp->kind) / (size_t)a.W;
       int64_t W = std::min<int64_t>({(int64_t)(kBatchWidth / a.tpt), (int64_t)a.G,
                                      (int64_t)std::max<size_t>(1, 110 * 1024 / per)});
       W = std::max<int64_t>(W, a.W);
@@ -1924,7 +1924,7 @@ std::unique_ptr<BatchProgram> lower_batch_t(const std::vector<BatchGroup> &group
         continue;
       a.W = (int)W;
       a.wdiv = make_fastdiv((uint32_t)W);
-      tp->smem = per * (size_t)W;
+      tp->smem = pp_tile_smem(a);  // of a launch on its own
     }
   size_t nph = 0;
   for (const auto &g : bp->groups) nph = std::max(nph, g.prog->passes.size());
@@ -1943,9 +1943,8 @@ std::unique_ptr<BatchProgram> lower_batch_t(const std::vector<BatchGroup> &group
                  : tp->kind == CoreKind::Rader     ? kBatchPpRader
                                                    : kBatchPpConv;
         }
-        // a persistent item runs the general ping-pong body: size its shared
-        // memory from the tile itself
-        const size_t item_smem = kind >= 0 && kind != kBatchRegcol ? pp_tile_smem(tp->a) : 0;
+        // size a persistent item's shared memory from the tile itself
+        const size_t item_smem = kind >= 0 && kind != kBatchRegcol ? batch_item_smem(tp->a, tp->kind) : 0;
         if (kind >= 0 && kind != kBatchRegcol && item_smem + kBatchSmemHeader > 232448) kind = -1;
         if (kind >= 0) {
           cls = batch_class(item_smem, tp->a.W * tp->a.tpt, kind == kBatchRegcol);

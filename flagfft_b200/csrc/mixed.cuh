@@ -36,10 +36,10 @@ namespace mixed {
 FFB_HD int buf_len(const Core &c) { return c.L + c.radix[0] + 1; }
 FFB_HD int slot_len(const Core &c, int nbuf) { return (nbuf * buf_len(c)) | 1; }
 
-// Buffers a pass needs: a two-stage complex transform writes shared memory
-// once; everything else alternates between two.
+// Buffers a pass needs: a complex transform of at most two stages writes
+// shared memory once; everything else alternates between two.
 FFB_HD int buffers(const Core &c, CoreKind kind, IoKind io) {
-  return kind == CoreKind::Dit && io == IoKind::C2C && c.nst == 2 ? 1 : 2;
+  return kind == CoreKind::Dit && io == IoKind::C2C && c.nst <= 2 ? 1 : 2;
 }
 
 template <typename T>
@@ -289,12 +289,13 @@ FFB_HD void twiddled_dft(cpx<T> (&v)[R], const cpx<T> *row, int Ns) {
   dft_fixed<R, INV, T>(v);
 }
 
-// All stages (two or more) of core c in direction INV: stage 0 reads through
-// src, the last writes through sink, the ones between alternate between the
-// two buffers; stage 0 writes buffer b.  wfast_in / wfast_out: consecutive
+// All stages of core c in direction INV: stage 0 reads through src, the last
+// writes through sink, the ones between alternate between the two buffers;
+// stage 0 writes buffer b.  A single codelet (batch programs) reads and
+// writes with nothing between.  wfast_in / wfast_out: consecutive
 // threads take consecutive transforms in the first / last stage (strided
 // layouts).  Returns the buffer the last stage read.
-template <bool INV, int SET, typename T, class X, class Src, class MakeSink>
+template <bool INV, int SET, typename T, bool SINGLE = false, class X, class Src, class MakeSink>
 FFB_HD void run_chain(const Tile<T> &t, const Core &c, const cpx<T> *__restrict__ tw, const X &x, const Src &src,
                       const MakeSink &make_sink, int b, bool wfast_in, bool wfast_out) {
   const TileArgs<T> &a = *t.a;
@@ -309,6 +310,23 @@ FFB_HD void run_chain(const Tile<T> &t, const Core &c, const cpx<T> *__restrict_
       j = e - w * nb;
     }
   };
+  if (S == 1) {
+    const auto sink = make_sink(b);
+#define FFB_MIXED_ONLY(R)                                       \
+  {                                                             \
+    _Pragma("unroll 1") for (int e = t0; e < W; e += nt) {      \
+      cpx<T> v[R];                                              \
+      src.template get<R>(e, 0, 1, v);                          \
+      dft_fixed<R, INV, T>(v);                                  \
+      sink.template put<R>(e, 0, 1, v);                         \
+    }                                                           \
+  }
+    if constexpr (SINGLE) {
+      FFB_MIXED_SWITCH(R0, FFB_MIXED_ONLY)
+    }
+#undef FFB_MIXED_ONLY
+    return;
+  }
   // stage 0: unit twiddles, output q of butterfly j at q * P0 + j
 #define FFB_MIXED_FIRST(R)                                        \
   {                                                               \
@@ -374,7 +392,7 @@ FFB_HD int last_buffer(const Core &c, int b) { return (c.nst & 1) ? 1 - b : b; }
 // One CTA tile of a pass: KIND 0 a Dit core in direction INV, 1 a fused
 // Bluestein, 2 a fused Rader, 3 a convolution row; REAL: any of the real
 // IoKinds (io), else complex in and out.
-template <typename T, int KIND, bool REAL, bool INV, int SET, class X>
+template <typename T, int KIND, bool REAL, bool INV, int SET, bool SINGLE = false, class X>
 FFB_HD void body(const TileArgs<T> &a, int io, long long bx, long long by, cpx<T> *sm, const X &x) {
   const bool real_in = REAL && (io == (int)IoKind::R2C || io == (int)IoKind::R2CFull);
   const bool real_out = REAL && (io == (int)IoKind::C2R || io == (int)IoKind::C2RFull);
@@ -431,7 +449,7 @@ FFB_HD void body(const TileArgs<T> &a, int io, long long bx, long long by, cpx<T
   const bool win = a.wfast != 0, wout = a.ok > a.og;
   const Source<T, KIND, REAL> src{&t, 0};
   if constexpr (KIND == 0) {
-    run_chain<INV, SET, T>(t, a.core, a.tw, x, src, [&](int ob) FFB_INL { return Sink<T, KIND, REAL>{&t, ob}; }, b, win,
+    run_chain<INV, SET, T, SINGLE>(t, a.core, a.tw, x, src, [&](int ob) FFB_INL { return Sink<T, KIND, REAL>{&t, ob}; }, b, win,
                       wout);
     b = 1 - last_buffer(a.core, b);  // where a shared-memory result is
   } else {

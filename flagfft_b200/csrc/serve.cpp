@@ -434,7 +434,7 @@ class Server {
                  : tp->kind == CoreKind::Rader     ? kBatchPpRader
                                                    : kBatchPpConv;
           // the request's own tile width (independent of the other requests)
-          const size_t per = pp_tile_smem(tp->a) / (size_t)tp->a.W;
+          const size_t per = batch_item_smem(tp->a, tp->kind) / (size_t)tp->a.W;
           if (a.tpt <= kBatchWidth) {
             int64_t W = std::min<int64_t>({(int64_t)(kBatchWidth / a.tpt), (int64_t)a.G,
                                            (int64_t)std::max<size_t>(1, 110 * 1024 / per)});
@@ -446,7 +446,10 @@ class Server {
             }
           }
           smem = per * (size_t)a.W;
-          if (smem + kBatchSmemHeader > 232448) kind = -1;
+          if (smem + kBatchSmemHeader > 232448) {
+            kind = -1;
+            smem = pp_tile_smem(a);  // of a launch on its own
+          }
         }
         if (kind < 0) {
           const CoreKind ck = tp->kind;
