@@ -577,11 +577,15 @@ class Builder {
     if (io == IoKind::C2C) {
       if (spec.kind == CoreKind::Dit && spec.radices.size() == 1) return {};
       if (fixed && spec.kind != CoreKind::Rader && ii == 1 && ok == 1) return {};
+      int tw = 0, th = 0;
+      size_t sm = 0;
       if (fixed && spec.kind == CoreKind::Dit && strided) {
-        int tw = 0, th = 0;
-        size_t sm = 0;
-        if (tiles_shape<T>((int)L, &tw, &th, &sm)) return {};
-        if (tma_columns_enabled() && tcols_eligible<T>((int)L, nbatch, G, ib, ig, ii, ob, og, ok, &th, &sm)) return {};
+        // (the column kernel's own sequence: it declines at launch when its
+        // tiles are too few, or its buffers break the copy rules)
+        if (tcols(spec, io, nbatch, G, ib, ig, ii, ob, og, ok, &th, &sm))
+          return nbatch <= 65535 && mixed_fits(spec, io, seq, 4) ? seq : std::vector<int>{};
+        // (a tile kernel with fewer CTAs than SMs leaves some idle)
+        if (tiles_shape<T>((int)L, &tw, &th, &sm) && nbatch * (G / tw) >= kSMs) return {};
       }
     } else if (io == IoKind::R2C ? (ii != 2 || ok != 1) : io == IoKind::C2R ? (ii != 1 || ok != 2)
                : io == IoKind::R2CFull || io == IoKind::C2RFull ? (ii != 1 || ok != 1) : true) {
@@ -590,13 +594,28 @@ class Builder {
     if (nbatch > 65535) return {};
     std::vector<int> r;
     if (!mixed_chain(L, 0, &r) && !mixed_chain(L, 1, &r)) return {};
-    if (r.size() < 2 || (int)r.size() > kMaxStages || L / r.front() < 4 || L / r.back() < 4) return {};
+    return mixed_fits(spec, io, r, 1) ? r : std::vector<int>{};
+  }
+
+  // W transforms of the chain fit one CTA and its global runs are long enough.
+  static bool mixed_fits(const CoreSpec &spec, IoKind io, const std::vector<int> &r, int W) {
+    const int64_t L = spec.L;
+    if (r.size() < 2 || (int)r.size() > kMaxStages || L / r.front() < 4 || L / r.back() < 4) return false;
     Core c{};
     c.L = (int)L;
     c.nst = (int)r.size();
     c.radix[0] = r[0];
-    const size_t per = ((size_t)mixed::slot_len(c, mixed::buffers(c, spec.kind, io)) + 2) * sizeof(cpx<T>);
-    return per <= 232448 ? r : std::vector<int>{};
+    return (size_t)W * ((size_t)mixed::slot_len(c, mixed::buffers(c, spec.kind, io)) + 2) * sizeof(cpx<T>) <= 232448;
+  }
+
+  // The column kernel takes the pass (tcols.cuh).
+  static bool tcols(const CoreSpec &spec, IoKind io, int64_t nbatch, int64_t G, long long ib, long long ig,
+                    long long ii, long long ob, long long og, long long ok, int *threads, size_t *smem) {
+    std::vector<int> seq, sorted_r = spec.radices;
+    std::sort(sorted_r.rbegin(), sorted_r.rend());
+    return spec.kind == CoreKind::Dit && io == IoKind::C2C && !t_no_one_pass && tma_columns_enabled() &&
+           fixed_sequence(spec.L, &seq) && seq == sorted_r &&
+           tcols_eligible<T>((int)spec.L, nbatch, G, ib, ig, ii, ob, og, ok, threads, smem);
   }
 
   // Cheapest chain of the radix set (stage_cost per element), largest first;
@@ -633,9 +652,12 @@ class Builder {
   static size_t choose_mixed(TileArgs<T> &a, CoreKind kind, IoKind io, bool strided) {
     const int regs = sizeof(T) == 4 ? (a.mixed_set == 0 ? 80 : 128) : (a.mixed_set == 0 ? 128 : 255);
     const int64_t most = std::min<int64_t>(a.G, 64);
+    // strided tiles move 64 bytes of a row, or 32 where that would leave SMs
+    // without a tile
     int64_t least = 1;
+    const int64_t wide = sizeof(T) == 4 ? 8 : 4;
     if (strided)
-      for (least = std::min<int64_t>(sizeof(T) == 4 ? 8 : 4, a.G);
+      for (least = std::min<int64_t>(a.nbatch * a.G / wide < kSMs ? wide / 2 : wide, a.G);
            least > 1 && mixed::smem_bytes(a, kind, io, (int)least) > 232448; --least) {
       }
     double best = 1e300;
@@ -746,6 +768,15 @@ class Builder {
       if (W_overflows(a.W, L, ig, ii) || W_overflows(a.W, L, og, ok))
         throw std::runtime_error("tile extent above 2^31 elements");
       a.tpt = 1;
+      {
+        int th = 0;
+        size_t sm = 0;
+        if (tcols(spec, io, nbatch, G, ib, ig, ii, ob, og, ok, &th, &sm)) {
+          a.tcols = 1;
+          a.tc_threads = th;
+          a.tc_smem = (int)sm;
+        }
+      }
       a.wdiv = make_fastdiv((uint32_t)a.W);
       a.pairs_div = make_fastdiv((uint32_t)(std::max<int64_t>(0, logical_n) / 2 / 2 + 1));
       p->kind = spec.kind;
@@ -804,9 +835,7 @@ class Builder {
     {
       int tc_threads = 0;
       size_t tc_smem = 0;
-      if (spec.kind == CoreKind::Dit && io == IoKind::C2C && a.pp && !t_no_one_pass && tma_columns_enabled() &&
-          fixed_sequence(L, &seq) && seq == sorted_r &&
-          tcols_eligible<T>((int)L, nbatch, G, ib, ig, ii, ob, og, ok, &tc_threads, &tc_smem)) {
+      if (a.pp && tcols(spec, io, nbatch, G, ib, ig, ii, ob, og, ok, &tc_threads, &tc_smem)) {
         a.tcols = 1;
         a.tc_threads = tc_threads;
         a.tc_smem = (int)tc_smem;

@@ -78,7 +78,7 @@ struct TilePass final : PassBase {
     for (int s = 0; s < a.core.nst; ++s) o << (s ? "," : "") << a.core.radix[s];
     o << "] n=" << a.n << " transforms=" << a.nbatch << "x" << a.G << " per_cta=" << a.W
       << " threads=" << (a.blue_cols ? blue4_threads(a.blue_cols, a.core.L, a.blue_pair != 0) : a.mixed ? a.mixed : a.tiles ? a.tpt : a.W * a.tpt)
-      << (a.tiles ? " tiles" : a.mixed ? " mixed" : "") << " smem=" << tile_smem<T>(a, kind, io, smem) << " " << buf_name(src) << "->"
+      << (a.tiles ? " tiles" : a.mixed ? " mixed tiles" : "") << " smem=" << tile_smem<T>(a, kind, io, smem) << " " << buf_name(src) << "->"
       << buf_name(dst);
     if (a.tcols) o << " tma-columns(threads=" << a.tc_threads << " smem=" << a.tc_smem << ")";
     if (a.post_twiddle) o << " +twiddle";

@@ -1,11 +1,12 @@
-// Instantiates the TMA column passes (tcols.cuh) in float precision.
-#include "tcols_impl.cuh"
+// Instantiates the TMA column passes (tcols.cuh, wcols.cuh) in float precision.
+#include "wcols_impl.cuh"
 
 namespace ffb {
 
 template <>
 cudaError_t launch_tcols<float>(const TileArgs<float> &a, cudaStream_t s) {
-  return tcols::launch_any<float>(a, s);
+  const cudaError_t e = wcols::launch_any(a, s);
+  return e == cudaErrorNotSupported ? tcols::launch_any<float>(a, s) : e;
 }
 
 template <>
@@ -17,9 +18,10 @@ bool tcols_eligible<float>(int L, long long nbatch, long long G, long long ib, l
 template <>
 long long tcols_wait_failures<float>() {
 #ifndef FFB_HOST_EMULATION
-  int v = 0;
+  int v = 0, w = 0;
   if (cudaMemcpyFromSymbol(&v, tcols::g_tcols_wait_failures, sizeof(int)) != cudaSuccess) return -1;
-  return v;
+  if (cudaMemcpyFromSymbol(&w, wcols::g_wcols_wait_failures, sizeof(int)) != cudaSuccess) return -1;
+  return (long long)v + w;
 #else
   return 0;
 #endif
