@@ -592,6 +592,10 @@ class Builder {
       return {};
     }
     if (nbatch > 65535) return {};
+    // (a half-length real pass of a compile-time sequence keeps it: the real
+    // row kernel takes it whenever its rows start on pairs)
+    if (fixed && spec.kind == CoreKind::Dit && (io == IoKind::R2C || io == IoKind::C2R))
+      return mixed_fits(spec, io, seq, 1) ? seq : std::vector<int>{};
     std::vector<int> r;
     if (!mixed_chain(L, 0, &r) && !mixed_chain(L, 1, &r)) return {};
     return mixed_fits(spec, io, r, 1) ? r : std::vector<int>{};

@@ -34,6 +34,12 @@ FFB_EXTERN(float)
 FFB_EXTERN(double)
 #undef FFB_EXTERN
 
+namespace rrows {
+// defined in k_*_rrows.cu
+template <typename T>
+cudaError_t launch(const TileArgs<T> &a, IoKind io, cudaStream_t s);
+}  // namespace rrows
+
 namespace mixed {
 // defined in k_*_mixed*.cu
 template <typename T, int K>
@@ -389,6 +395,10 @@ cudaError_t launch_tile(const TileArgs<T> &a, CoreKind kind, IoKind io, size_t s
     if (e != cudaErrorNotSupported) return e;  // else: buffers off the copy rules, the tile kernels below
   }
   if (a.tiles) return launch_tiles<T>(a, s);
+  if (k == 0 && (o == 1 || o == 2)) {
+    const cudaError_t e = rrows::launch<T>(a, io, s);
+    if (e != cudaErrorNotSupported) return e;  // else: no compile-time sequence, or rows off pairs
+  }
   if (a.mixed) {
     switch (k) {
       case 0: return mixed::launch<T, 0>(a, io, smem, s);
