@@ -20,6 +20,7 @@
 #pragma once
 
 #include <atomic>
+#include <type_traits>
 
 #include "rows.cuh"
 
@@ -28,9 +29,59 @@ namespace blue4 {
 
 using rows::Seq;
 using rows::SmemIO;
-using rows::SmemKernIO;
 using rows::slot_len;
 using rows::tpt_of;
+
+// A sequence with its radices in reverse order: the convolution's inverse
+// core.  Its first stage takes elements j + r L/R of butterfly j, R the
+// forward core's last radix -- the outputs of the forward core's last
+// butterfly j -- so the kernel product and that stage happen in the registers
+// of the forward stage's threads (FusedIO).
+template <class Q>
+struct Reversed {
+  static constexpr int n = Q::n;
+  static FFB_HD constexpr int r(int s) { return Q::r(n - 1 - s); }
+  static FFB_HD constexpr int span(int s) {
+    int p = 1;
+    for (int i = 0; i < s; ++i) p *= r(i);
+    return p;
+  }
+  static FFB_HD constexpr int twoff(int s) {
+    int o = 0;
+    for (int i = 0; i < s; ++i) o += (r(i) - 1) * span(i);
+    return o;
+  }
+};
+template <int L, int... Rs>
+FFB_HD bool core_is_reversed(const Core &c) {
+  using Q = Reversed<Seq<Rs...>>;
+  if (c.L != L || c.nst != Q::n) return false;
+  for (int s = 0; s < Q::n; ++s)
+    if (c.radix[s] != Q::r(s)) return false;
+  return true;
+}
+
+// Last forward stage of a row: output k (natural order) times the kernel
+// spectrum entry k, then the first stage of the inverse core on the same
+// registers, its outputs into the row's buffer.  Against a product written in
+// natural order and a first inverse stage of its own this saves one of the
+// five shared-memory round trips and two barriers of a row: C2C 10007 x 1024
+// 162.2 -> 156.4 us on one B200.  (The row kernels of rows.cuh, several CTAs
+// per SM, gain nothing: C2C 1009 x 1024 12.1 -> 12.3, Z2Z 10007 x 256 103.5 ->
+// 106.8, so they keep the stage apart.)
+template <typename T>
+struct FusedIO {
+  cpx<T> *b;
+  const cpx<T> *kern;
+  template <int S, int R>
+  FFB_HD void put(int base, const cpx<T> (&x)[R]) const {
+    cpx<T> y[R];
+#pragma unroll
+    for (int q = 0; q < R; ++q) y[q] = cmul(x[q], ldg_c(kern + base + q * S));
+    dft_fixed<R, true, T>(y);
+    SmemIO<T>{b}.template put<1, R>(base * R, y);  // (base is the butterfly's index)
+  }
+};
 
 // W_M^m (forward sign) from the pass's two split four-step tables, m < M.
 template <typename T>
@@ -50,9 +101,10 @@ struct Shape {
   static constexpr int slot = slot_len<L2>();
 };
 
-// The row convolution as one pipeline of 2 x nst stages (nst forward, then
-// nst inverse; the last forward stage multiplies by the kernel spectrum row)
-// over two groups of rows.  Step k reads group k % 2 of stage k / 2; between
+// The row convolution as one pipeline of 2 x nst - 1 stages (nst forward, then
+// nst - 1 inverse ones of the reversed sequence: the last forward stage
+// multiplies by the kernel spectrum row and runs the inverse's first stage in
+// its registers) over two groups of rows.  Step k reads group k % 2 of stage k / 2; between
 // two barriers a thread writes what it read in the previous step and reads
 // the next group:  R(0,0) | W(0,0) R(0,1) | W(0,1) R(1,0) | ... | W(last,1).
 // A write and the read after it touch different row groups, and every read
@@ -62,8 +114,9 @@ template <typename T, int N1, int L2, class Q, class Sh, int S>
 struct RowStage {
   static constexpr int nst = Q::n;
   static constexpr bool inv = S >= nst;
-  static constexpr int qs = inv ? S - nst : S;
-  static constexpr int R = Q::r(qs), Ns = Q::span(qs), TwOff = Q::twoff(qs);
+  static constexpr int qs = inv ? S - nst + 1 : S;
+  using QS = std::conditional_t<inv, Reversed<Q>, Q>;
+  static constexpr int R = QS::r(qs), Ns = QS::span(qs), TwOff = QS::twoff(qs);
   using Regs = rows::StageRegs<T, L2, Sh::TPT, R>;
 
   static FFB_HD Regs read(const TileArgs<T> &a, cpx<T> *sm, int grp, int tid) {
@@ -75,7 +128,7 @@ struct RowStage {
     const int w = grp * Sh::NR + tid / Sh::TPT, t = tid % Sh::TPT;
     if (w >= N1) return;
     if constexpr (S == nst - 1) {
-      rows::stage_write<T, L2, Sh::TPT, Ns, R>(t, st, SmemKernIO<T>{sm + w * Sh::slot, kern + w * a.kern_stride});
+      rows::stage_write<T, L2, Sh::TPT, Ns, R>(t, st, FusedIO<T>{sm + w * Sh::slot, kern + w * a.kern_stride});
     } else {
       rows::stage_write<T, L2, Sh::TPT, Ns, R>(t, st, SmemIO<T>{sm + w * Sh::slot});
     }
@@ -90,7 +143,7 @@ FFB_HD void row_pipe(const X &x, const TileArgs<T> &a, cpx<T> *sm, const cpx<T> 
   static_assert(Sh::NG == 2, "the pipeline runs two row groups");
   constexpr int P = K - 1;  // the step whose reads st holds
   using Prev = RowStage<T, N1, L2, Q, Sh, P / 2>;
-  if constexpr (K == 4 * Q::n) {
+  if constexpr (K == 2 * (2 * Q::n - 1)) {
     x.last(Sh::NT, [&](int tid, const typename Prev::Regs &s) FFB_INL { Prev::write(a, sm, kern, P % 2, tid, s); }, st);
   } else {
     using Cur = RowStage<T, N1, L2, Q, Sh, K / 2>;

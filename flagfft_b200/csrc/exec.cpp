@@ -728,8 +728,10 @@ class Builder {
     if (!mixed_r.empty()) a.pp = 1;
     // ping-pong cores run their radices largest first (any order is the same
     // DFT; this one matches the compile-time sequences), and a convolution's
-    // inverse core the same order; the in-place pair needs DIF then DIT with
-    // the radices reversed
+    // inverse core the same order on the row kernels and reversed elsewhere
+    // (the mixed-radix tiles, which batch programs run too, join its first
+    // stage to the forward core's last; the in-place pair needs DIF then DIT
+    // with the radices reversed)
     std::vector<int> radices = mixed_r.empty() ? spec.radices : mixed_r;
     if (a.pp) std::sort(radices.rbegin(), radices.rend());
     if (spec.kind == CoreKind::Dit) {
@@ -737,7 +739,8 @@ class Builder {
     } else {
       a.core = a.pp ? make_dit_core(L, radices) : make_dif_core(L, radices);
       std::vector<int> rev(radices.rbegin(), radices.rend());
-      a.core2 = make_dit_core(L, a.pp ? radices : rev);
+      const bool row_kernel = a.pp && mixed_r.empty() && !t_no_one_pass;
+      a.core2 = make_dit_core(L, row_kernel ? radices : rev);
       if (spec.kind != CoreKind::Conv) fill_convolution(a, spec, inverse);  // Conv: caller supplies the kernel
     }
     // one-codelet transforms lying side by side in memory on both sides run
@@ -1309,6 +1312,8 @@ void lower_c2c(Builder<T> &bld, Program &prog, const NodePtr &root, bool inverse
       a.chirp = bld.table_chirp(n, inverse);
       a.kern = bld.table_bluestein_rows(n, row_radices, n1, n2, inverse, true);
       a.kern_stride = n2;
+      a.core2 = make_dit_core(n2, std::vector<int>(row_radices.rbegin(), row_radices.rend()));
+      a.tw2 = bld.table_stage_twiddles(a.core2, false, true);
       bld.set_post_twiddle(a, M);
       p->smem = blue4_smem((int)n1, (int)n2, sizeof(cpx<T>), pair);
       p->note = "bluestein one pass: " + std::to_string(n1) + " x " + std::to_string(n2) +

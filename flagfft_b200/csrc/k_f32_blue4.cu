@@ -7,13 +7,13 @@ template <>
 cudaError_t launch_blue4<float>(const TileArgs<float> &a, cudaStream_t s) {
 #define FFB_B4_LAUNCH(N1, L2, ...)                                                                                   \
   if (!a.blue_pair && a.blue_cols == (N1) && tile::core_is<L2, __VA_ARGS__>(a.core) &&                             \
-      tile::core_is<L2, __VA_ARGS__>(a.core2))                                                                     \
+      blue4::core_is_reversed<L2, __VA_ARGS__>(a.core2))                                                                     \
     return blue4::launch<float, N1, L2, __VA_ARGS__>(a, s);
   FFB_BLUE4_SHAPES(FFB_B4_LAUNCH)
 #undef FFB_B4_LAUNCH
 #define FFB_B4P_LAUNCH(N1, L2, ...)                                                                                  \
   if (a.blue_pair && a.blue_cols == (N1) && tile::core_is<L2, __VA_ARGS__>(a.core) &&                              \
-      tile::core_is<L2, __VA_ARGS__>(a.core2))                                                                     \
+      blue4::core_is_reversed<L2, __VA_ARGS__>(a.core2))                                                                     \
     return blue4::launch_pair<float, N1, L2, __VA_ARGS__>(a, s);
   FFB_BLUE4_PAIR_SHAPES(FFB_B4P_LAUNCH)
 #undef FFB_B4P_LAUNCH

@@ -18,11 +18,16 @@
 //   * packs a real transform's pairs on its load or store and does the
 //     Hermitian post / pre step from shared memory, both bins of a pair (k,
 //     n/2 - k) from one twiddle.
+// A convolution's inverse chain runs the radices reversed, so that its first
+// stage happens in the registers of the forward chain's last: one of its
+// round trips less.
 // Measured on one B200 against the ping-pong and in-place bodies these passes
 // ran on before: C2C 1200 x 4096 inverse 70.7 -> 25.7 us (3.1 TB/s of input
-// and output), R2C + C2R 2048 x 8192 254 -> 103 us, D2Z + Z2D 1500 x 1024
-// 42.9 -> 24.9 us.  What bounds it now is the shared-memory and codelet
-// instruction stream of 16 to 24 warps per SM, not HBM.
+// and output), D2Z + Z2D 1500 x 1024 42.9 -> 24.9 us; the joined stages took
+// 600 uneven transforms in one batch plan from 113.2 to 109.3 us.  What bounds
+// it now is the shared-memory and codelet instruction stream of 16 to 24 warps
+// per SM, not HBM: over ten tile shapes and four radix chains the two calls
+// above moved by 2% from the shape choose_mixed takes (exec.cpp).
 #pragma once
 
 #include "tile_impl.cuh"
@@ -227,21 +232,11 @@ struct Sink {
   }
 };
 
-// A stage's input from shared memory (natural order): elements j + r * nb.
-template <typename T>
-struct SmemSource {
-  const Tile<T> *t;
-  int b;
-  template <int R>
-  FFB_HD void get(int w, int j, int nb, cpx<T> (&v)[R]) const {
-    const cpx<T> *p = t->buf(w, b) + j;
-#pragma unroll
-    for (int r = 0; r < R; ++r) v[r] = p[r * nb];
-  }
-};
-
 // The forward chain's last stage of a convolution: times the kernel spectrum
-// (natural order), into shared memory; a Rader core's X0 = x0 + DC on the way.
+// (natural order), then the inverse chain's first stage -- its radices are the
+// forward chain's reversed, so butterfly j takes the same R values -- into
+// shared memory in that stage's transposed layout; a Rader core's X0 = x0 +
+// DC on the way.
 template <typename T, int KIND>
 struct KernelSink {
   const Tile<T> *t;
@@ -255,8 +250,12 @@ struct KernelSink {
     if constexpr (KIND == 2) {
       if (j == 0) t->extra[a.W + w] = v[0] + t->extra[w];
     }
+    cpx<T> y[R];
 #pragma unroll
-    for (int q = 0; q < R; ++q) p[q * nb] = cmul(v[q], ldg_c(kern + j + q * nb));
+    for (int q = 0; q < R; ++q) y[q] = cmul(v[q], ldg_c(kern + j + q * nb));
+    dft_fixed<R, true, T>(y);
+#pragma unroll
+    for (int q = 0; q < R; ++q) p[q * (nb | 1)] = y[q];
   }
 };
 
@@ -294,8 +293,8 @@ FFB_HD void twiddled_dft(cpx<T> (&v)[R], const cpx<T> *row, int Ns) {
 // stage 0 writes buffer b.  A single codelet (batch programs) reads and
 // writes with nothing between.  wfast_in / wfast_out: consecutive
 // threads take consecutive transforms in the first / last stage (strided
-// layouts).  Returns the buffer the last stage read.
-template <bool INV, int SET, typename T, bool SINGLE = false, class X, class Src, class MakeSink>
+// layouts).  START = 1: stage 0 is already in buffer b.
+template <bool INV, int SET, typename T, bool SINGLE = false, int START = 0, class X, class Src, class MakeSink>
 FFB_HD void run_chain(const Tile<T> &t, const Core &c, const cpx<T> *__restrict__ tw, const X &x, const Src &src,
                       const MakeSink &make_sink, int b, bool wfast_in, bool wfast_out) {
   const TileArgs<T> &a = *t.a;
@@ -340,9 +339,11 @@ FFB_HD void run_chain(const Tile<T> &t, const Core &c, const cpx<T> *__restrict_
       _Pragma("unroll") for (int q = 0; q < R; ++q) p[q * P0] = v[q]; \
     }                                                             \
   }
-  FFB_MIXED_SWITCH(R0, FFB_MIXED_FIRST)
+  if constexpr (START == 0) {
+    FFB_MIXED_SWITCH(R0, FFB_MIXED_FIRST)
+    x.sync();
+  }
 #undef FFB_MIXED_FIRST
-  x.sync();
   for (int s = 1; s < S - 1; ++s) {
     const int Ns = c.span[s];
     const cpx<T> *blk = tw + c.twoff[s];
@@ -456,11 +457,10 @@ FFB_HD void body(const TileArgs<T> &a, int io, long long bx, long long by, cpx<T
     run_chain<false, SET, T>(t, a.core, a.tw, x, src, [&](int ob) FFB_INL { return KernelSink<T, KIND>{&t, ob}; }, b, win,
                         false);
     x.sync();
-    b = 1 - last_buffer(a.core, b);  // the product
-    const SmemSource<T> ps{&t, b};
-    run_chain<true, SET, T>(t, a.core2, a.tw2, x, ps, [&](int ob) FFB_INL { return Sink<T, KIND, REAL>{&t, ob}; }, 1 - b,
-                       false, wout);
-    b = 1 - last_buffer(a.core2, 1 - b);
+    b = 1 - last_buffer(a.core, b);  // the product, through the inverse chain's first stage
+    run_chain<true, SET, T, false, 1>(t, a.core2, a.tw2, x, src,
+                                      [&](int ob) FFB_INL { return Sink<T, KIND, REAL>{&t, ob}; }, b, false, wout);
+    b = 1 - last_buffer(a.core2, b);
     if constexpr (KIND == 2) {
       for (int w = t0; w < t.wlive; w += nt) put_result<T, REAL>(t, w, 0, t.extra[W + w], t.buf(w, b));
     }
