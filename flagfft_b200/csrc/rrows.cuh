@@ -11,7 +11,7 @@
 // keeps one buffer instead of two.
 //
 // Measured on one B200 (in-place tiles, mixed-radix tiles, here): R2C + C2R
-// 2048 x 8192 254 -> 103 -> 62.8 us (4.3 TB/s of input and output); 512 x 10000
+// 2048 x 8192 254 -> 103 -> 60.2 us (4.5 TB/s of input and output); 512 x 10000
 // forward 37.7 -> 8.9 here.  What bounds it is the Hermitian step's extra round
 // trip through shared memory.
 #pragma once
@@ -144,11 +144,23 @@ cudaError_t launch_seq(const TileArgs<T> &a, cudaStream_t s) {
       1, std::min<long long>({128 / TPT, (long long)(110 * 1024 / per), a.nbatch * a.G / (2 * 148), (long long)a.G}));
   const long long tiles = (a.G + W - 1) / W;
 #ifndef FFB_HOST_EMULATION
+  const dim3 grid((unsigned)tiles, (unsigned)a.nbatch), block((unsigned)(W * TPT));
+  // many rows: the 64-register form (rows.cuh rows_dense says when and why).
+  // Measured (us, R2C / C2R): 2048 x 8192 31.0 / 35.1 -> 29.5 / 32.8, 8192 x 1024
+  // 18.5 / 24.6 -> 17.3 / 19.1, 16384 x 512 27.1 / 31.4 -> 22.5 / 25.7; 1024 x 64
+  // 4.2 / 4.6 -> 6.2 / 6.3, 3072 x 2000 14.2 / 14.5 -> 17.9 / 16.9
+  constexpr bool dense = sizeof(T) == 4 && (L & (L - 1)) == 0 && L >= 512 && L <= 8192;
+  if constexpr (dense) {
+    if (a.nbatch * a.G * (long long)L >= rows::kDensePoints) {
+      cudaError_t e = set_smem_limit_once<k_rrows<T, INV, 2, L, TPT, Rs...>>(232448);
+      if (e != cudaSuccess) return e;
+      return launch_pdl(k_rrows<T, INV, 2, L, TPT, Rs...>, grid, block, (size_t)W * per, s, a, (int)W);
+    }
+  }
   constexpr int MB = rows::rows_min_blocks<T, 0, L>();
   cudaError_t e = set_smem_limit_once<k_rrows<T, INV, MB, L, TPT, Rs...>>(232448);
   if (e != cudaSuccess) return e;
-  return launch_pdl(k_rrows<T, INV, MB, L, TPT, Rs...>, dim3((unsigned)tiles, (unsigned)a.nbatch),
-                    dim3((unsigned)(W * TPT)), (size_t)W * per, s, a, (int)W);
+  return launch_pdl(k_rrows<T, INV, MB, L, TPT, Rs...>, grid, block, (size_t)W * per, s, a, (int)W);
 #else
   (void)s;
   std::vector<unsigned char> buf((size_t)W * per + 64);
