@@ -728,10 +728,11 @@ class Builder {
     if (!mixed_r.empty()) a.pp = 1;
     // ping-pong cores run their radices largest first (any order is the same
     // DFT; this one matches the compile-time sequences), and a convolution's
-    // inverse core the same order on the row kernels and reversed elsewhere
-    // (the mixed-radix tiles, which batch programs run too, join its first
-    // stage to the forward core's last; the in-place pair needs DIF then DIT
-    // with the radices reversed)
+    // inverse core the same order on the row kernels (which a pass that only
+    // they can hold takes in a batch program too: it launches on its own) and
+    // reversed elsewhere (the mixed-radix tiles, which batch programs run
+    // too, join its first stage to the forward core's last; the in-place pair
+    // needs DIF then DIT with the radices reversed)
     std::vector<int> radices = mixed_r.empty() ? spec.radices : mixed_r;
     if (a.pp) std::sort(radices.rbegin(), radices.rend());
     if (spec.kind == CoreKind::Dit) {
@@ -739,7 +740,7 @@ class Builder {
     } else {
       a.core = a.pp ? make_dit_core(L, radices) : make_dif_core(L, radices);
       std::vector<int> rev(radices.rbegin(), radices.rend());
-      const bool row_kernel = a.pp && mixed_r.empty() && !t_no_one_pass;
+      const bool row_kernel = a.pp && mixed_r.empty() && (!t_no_one_pass || a.rows_only);
       a.core2 = make_dit_core(L, row_kernel ? radices : rev);
       if (spec.kind != CoreKind::Conv) fill_convolution(a, spec, inverse);  // Conv: caller supplies the kernel
     }

@@ -100,3 +100,20 @@ def test_batch_without_graphs(ffb, torch_cuda, monkeypatch):
         _check_groups(b.cpu().numpy(), x, lengths, counts, 1, False)
     finally:
         plan.destroy()
+
+
+# convolution rows of one CTA each (8192 points double, 16384 single): the
+# row kernel launches them on its own beside the persistent launches
+@pytest.mark.parametrize("lengths,counts,double", [([33013, 1701, 40009, 65521], [2, 3, 1, 1], True),
+                                                   ([65539, 1701, 100003, 131071], [2, 3, 1, 1], False)],
+                         ids=["Z2Z", "C2C"])
+def test_batch_convolution_rows_of_one_cta(ffb, torch_cuda, lengths, counts, double):
+    total = sum(n * c for n, c in zip(lengths, counts))
+    x = O.random_complex(total, 33, double)
+    plan = ffb.plan_batch(lengths, counts, ffb.Z2Z if double else ffb.C2C)
+    try:
+        for direction in (-1, 1):
+            _, b = _run(ffb, torch_cuda, plan, x, direction)
+            _check_groups(b.cpu().numpy(), x, lengths, counts, direction, double)
+    finally:
+        plan.destroy()

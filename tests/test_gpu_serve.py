@@ -171,3 +171,25 @@ def test_server_wait_timeout_keeps_ticket(ffb, torch_cuda):
     ref = np.fft.fft(x.cpu().numpy().astype(np.complex128), axis=-1)
     err = O.error_stats(y.cpu().numpy(), ref)
     assert err["rel_l2"] <= O.north_star_bound(O.C2C, n)
+
+
+def test_server_convolution_rows_of_one_cta(ffb, torch_cuda):
+    """Requests whose convolution rows fill a CTA (Z2Z primes above 32768,
+    C2C primes above 65536) launch those on their own, in the same tick as
+    shorter requests."""
+    torch = torch_cuda
+    reqs = []
+    for k, (t, n, b, d) in enumerate([("Z2Z", 33013, 2, -1), ("Z2Z", 65521, 1, 1), ("C2C", 100003, 1, -1),
+                                      ("C2C", 131071, 1, 1), ("C2C", 1701, 3, 1), ("Z2Z", 4096, 2, -1)]):
+        x = O.random_complex(n * b, 71 + k, t == "Z2Z").reshape(b, n)
+        xd = torch.from_numpy(x).cuda()
+        reqs.append((t, n, b, d, x, xd, torch.empty_like(xd)))
+    with ffb.Server(hbm_budget_bytes=4 << 30, max_ticks=2) as srv:
+        for t, n, b, d, *_ in reqs:
+            srv.prepare(getattr(ffb, t), n, d)
+        tickets = [srv.submit(getattr(ffb, t), n, b, xd, yd, d) for t, n, b, d, x, xd, yd in reqs]
+        for tk in tickets:
+            srv.wait(tk, timeout_s=60.0)
+    for t, n, b, d, x, xd, yd in reqs:
+        err = O.error_stats(yd.cpu().numpy(), O.c2c(x.astype(np.complex128), d))
+        assert err["finite"] and err["rel_l2"] <= O.north_star_bound(getattr(O, t), n), (t, n, b, d, err)

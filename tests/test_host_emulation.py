@@ -208,3 +208,55 @@ def test_server_real_on_chip_items():
     assert _rel(outs[1], np.stack([O.c2r(r.astype(np.complex128), n2) for r in x2])) < _bound(n2, False)
     assert _rel(outs[2], np.stack([O.r2c(r) for r in x3])) < _bound(n3, True)
     assert _rel(outs[3], np.stack([O.c2r(r, n3) for r in x4])) < _bound(n3, True)
+
+
+def _batch_run(lengths, counts, x, direction, double):
+    """One batch plan over the packed groups; returns its output."""
+    import ctypes
+    L = H.lib()
+    i = ctypes.c_int
+    L.flagfftB200PlanBatch.argtypes = [ctypes.POINTER(ctypes.c_void_p), i, ctypes.POINTER(i), ctypes.POINTER(i), i]
+    g = len(lengths)
+    h = ctypes.c_void_p()
+    assert L.flagfftB200PlanBatch(ctypes.byref(h), g, (i * g)(*lengths), (i * g)(*counts), Z2Z if double else C2C) == 0
+    y = np.empty_like(x)
+    try:
+        assert (L.flagfftExecZ2Z if double else L.flagfftExecC2C)(h, H._p(x), H._p(y), direction) == 0
+    finally:
+        L.flagfftDestroy(h)
+    return y
+
+
+def _check_batch(lengths, counts, double):
+    total = sum(n * c for n, c in zip(lengths, counts))
+    x = O.random_complex(total, total, double=True).astype(np.complex128 if double else np.complex64)
+    for direction in (-1, 1):
+        y = _batch_run(lengths, counts, x, direction, double)
+        at = 0
+        for n, c in zip(lengths, counts):
+            xs = x[at:at + n * c].reshape(c, n).astype(np.complex128)
+            assert _rel(y[at:at + n * c], O.c2c(xs, direction)) < _bound(n, double), (n, direction)
+            at += n * c
+
+
+# convolution rows of one CTA each (8192 points double, 16384 single): the
+# row kernel launches them on its own beside the persistent launches
+@pytest.mark.parametrize("lengths,double", [([33013], True), ([40009, 1701], True), ([65521], True),
+                                            ([65539], False), ([1701, 100003], False), ([131071], False)])
+def test_batch_convolution_rows_of_one_cta(lengths, double):
+    _check_batch(lengths, [1] * len(lengths), double)
+
+
+def test_server_convolution_rows_of_one_cta():
+    """Requests whose convolution rows launch on their own, beside shorter
+    ones of the same tick; a real one that widens to such a length."""
+    reqs, kinds = [], [(Z2Z, 40009, 1, -1), (Z2Z, 65521, 1, 1), (C2C, 100003, 1, -1), (C2C, 1701, 2, 1),
+                       (C2C, 4096, 1, -1), (Z2Z, 1701, 1, -1)]
+    for k, (code, n, b, d) in enumerate(kinds):
+        x = O.random_complex(n * b, 61 + k, double=True).reshape(b, n)
+        reqs.append((code, n, b, d, x.astype(np.complex128 if code == Z2Z else np.complex64)))
+    r = O.random_real(33013, 71, True).reshape(1, 33013).astype(np.float64)
+    outs = _server_run(reqs + [(D2Z, 33013, 1, -1, r)])
+    for (code, n, b, d, x), y in zip(reqs, outs):
+        assert _rel(y, O.c2c(x.astype(np.complex128), d)) < _bound(n, code == Z2Z), (code, n)
+    assert _rel(outs[-1], O.r2c(r)) < _bound(33013, True)
