@@ -467,6 +467,9 @@ class Builder {
 
   static constexpr int kMaxThreads = sizeof(T) == 4 ? 512 : 256;
   static constexpr int64_t kSMs = 148;
+  // Shared memory of one SM, and what the system takes of it for each CTA: a
+  // CTA of the most one may have (232448 bytes) still fits.
+  static constexpr size_t kSmSmem = 233472, kCtaSmem = 1024;
 
   // Two ping-pong buffers of a length-L transform fit one CTA.
   static bool pp_fits(int64_t L) {
@@ -669,7 +672,8 @@ class Builder {
       for (int64_t W = least; W <= most; ++W) {
         const size_t smem = mixed::smem_bytes(a, kind, io, (int)W);
         if (smem > 232448) break;
-        const int64_t per_sm = std::min<int64_t>({65536 / (regs * NT), (int64_t)(232448 / (smem + 1024)), 2048 / NT, 32});
+        const int64_t per_sm =
+            std::min<int64_t>({65536 / (regs * NT), (int64_t)(kSmSmem / (smem + kCtaSmem)), 2048 / NT, 32});
         if (per_sm < 1) continue;
         const int64_t tiles = a.nbatch * ((a.G + W - 1) / W);
         double issue = 0, latency = 2000;
