@@ -130,7 +130,7 @@ FFB_HD void run_item(const TileArgs<T> &a, int kind, int tile, cpx<T> *sm, const
   } else if (kind == kBatchPpRader) {
     mixed::body<T, 2, false, false, 1>(a, 0, bx, by, sm, x);
   } else {
-    mixed::body<T, 3, false, false, 1>(a, 0, bx, by, sm, x);
+    mixed::body<T, 3, false, false, 1, true>(a, 0, bx, by, sm, x);
   }
 }
 

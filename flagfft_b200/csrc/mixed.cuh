@@ -290,10 +290,11 @@ FFB_HD void twiddled_dft(cpx<T> (&v)[R], const cpx<T> *row, int Ns) {
 
 // All stages of core c in direction INV: stage 0 reads through src, the last
 // writes through sink, the ones between alternate between the two buffers;
-// stage 0 writes buffer b.  A single codelet (batch programs) reads and
-// writes with nothing between.  wfast_in / wfast_out: consecutive
-// threads take consecutive transforms in the first / last stage (strided
-// layouts).  START = 1: stage 0 is already in buffer b.
+// stage 0 writes buffer b.  A single codelet (SINGLE: batch programs, whose
+// convolution rows may be one too) reads and writes with nothing between.
+// wfast_in / wfast_out: consecutive threads take consecutive transforms in the
+// first / last stage (strided layouts).  START = 1: stage 0 is already in
+// buffer b.
 template <bool INV, int SET, typename T, bool SINGLE = false, int START = 0, class X, class Src, class MakeSink>
 FFB_HD void run_chain(const Tile<T> &t, const Core &c, const cpx<T> *__restrict__ tw, const X &x, const Src &src,
                       const MakeSink &make_sink, int b, bool wfast_in, bool wfast_out) {
@@ -310,20 +311,25 @@ FFB_HD void run_chain(const Tile<T> &t, const Core &c, const cpx<T> *__restrict_
     }
   };
   if (S == 1) {
-    const auto sink = make_sink(b);
-#define FFB_MIXED_ONLY(R)                                       \
-  {                                                             \
-    _Pragma("unroll 1") for (int e = t0; e < W; e += nt) {      \
-      cpx<T> v[R];                                              \
-      src.template get<R>(e, 0, 1, v);                          \
-      dft_fixed<R, INV, T>(v);                                  \
-      sink.template put<R>(e, 0, 1, v);                         \
-    }                                                           \
-  }
     if constexpr (SINGLE) {
+      const auto sink = make_sink(b);
+#define FFB_MIXED_ONLY(R)                                                       \
+  {                                                                             \
+    _Pragma("unroll 1") for (int e = t0; e < W; e += nt) {                      \
+      cpx<T> v[R];                                                              \
+      if constexpr (START == 0) {                                               \
+        src.template get<R>(e, 0, 1, v);                                        \
+        dft_fixed<R, INV, T>(v);                                                \
+      } else {                                                                  \
+        const cpx<T> *p = t.buf(e, b);                                          \
+        _Pragma("unroll") for (int r = 0; r < R; ++r) v[r] = p[r];              \
+      }                                                                         \
+      sink.template put<R>(e, 0, 1, v);                                         \
+    }                                                                           \
+  }
       FFB_MIXED_SWITCH(R0, FFB_MIXED_ONLY)
-    }
 #undef FFB_MIXED_ONLY
+    }
     return;
   }
   // stage 0: unit twiddles, output q of butterfly j at q * P0 + j
@@ -454,12 +460,12 @@ FFB_HD void body(const TileArgs<T> &a, int io, long long bx, long long by, cpx<T
                       wout);
     b = 1 - last_buffer(a.core, b);  // where a shared-memory result is
   } else {
-    run_chain<false, SET, T>(t, a.core, a.tw, x, src, [&](int ob) FFB_INL { return KernelSink<T, KIND>{&t, ob}; }, b, win,
-                        false);
+    run_chain<false, SET, T, SINGLE>(t, a.core, a.tw, x, src,
+                                     [&](int ob) FFB_INL { return KernelSink<T, KIND>{&t, ob}; }, b, win, false);
     x.sync();
     b = 1 - last_buffer(a.core, b);  // the product, through the inverse chain's first stage
-    run_chain<true, SET, T, false, 1>(t, a.core2, a.tw2, x, src,
-                                      [&](int ob) FFB_INL { return Sink<T, KIND, REAL>{&t, ob}; }, b, false, wout);
+    run_chain<true, SET, T, SINGLE, 1>(t, a.core2, a.tw2, x, src,
+                                       [&](int ob) FFB_INL { return Sink<T, KIND, REAL>{&t, ob}; }, b, false, wout);
     b = 1 - last_buffer(a.core2, b);
     if constexpr (KIND == 2) {
       for (int w = t0; w < t.wlive; w += nt) put_result<T, REAL>(t, w, 0, t.extra[W + w], t.buf(w, b));

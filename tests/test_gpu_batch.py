@@ -117,3 +117,19 @@ def test_batch_convolution_rows_of_one_cta(ffb, torch_cuda, lengths, counts, dou
             _check_groups(b.cpu().numpy(), x, lengths, counts, direction, double)
     finally:
         plan.destroy()
+
+
+@pytest.mark.parametrize("double", [False, True], ids=["C2C", "Z2Z"])
+def test_batch_convolution_rows_of_one_codelet(ffb, torch_cuda, monkeypatch, double):
+    """Short primes split over three passes: convolution rows of 3 to 19 points."""
+    monkeypatch.setenv("FLAGFFT_ONCHIP_POLICY", "multipass")
+    lengths, counts = [23, 53, 4, 97, 1009, 211], [300, 1, 2, 50, 1, 20]
+    total = sum(n * c for n, c in zip(lengths, counts))
+    x = O.random_complex(total, 47, double)
+    plan = ffb.plan_batch(lengths, counts, ffb.Z2Z if double else ffb.C2C)
+    try:
+        for direction in (-1, 1):
+            _, b = _run(ffb, torch_cuda, plan, x, direction)
+            _check_groups(b.cpu().numpy(), x, lengths, counts, direction, double)
+    finally:
+        plan.destroy()

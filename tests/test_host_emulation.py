@@ -260,3 +260,15 @@ def test_server_convolution_rows_of_one_cta():
     for (code, n, b, d, x), y in zip(reqs, outs):
         assert _rel(y, O.c2c(x.astype(np.complex128), d)) < _bound(n, code == Z2Z), (code, n)
     assert _rel(outs[-1], O.r2c(r)) < _bound(33013, True)
+
+
+# convolution rows of one codelet (a prime split over three passes)
+@pytest.mark.parametrize("double", [False, True])
+def test_batch_convolution_rows_of_one_codelet(monkeypatch, double):
+    monkeypatch.setenv("FLAGFFT_ONCHIP_POLICY", "multipass")
+    _check_batch([23, 53, 4, 97, 1009, 211], [3, 1, 2, 5, 1, 2], double)
+    outs = _server_run([(Z2Z if double else C2C, 29, 3, d, O.random_complex(87, 5, double).reshape(3, 29))
+                        for d in (-1, 1)])
+    for d, y in zip((-1, 1), outs):
+        ref = O.c2c(O.random_complex(87, 5, double).reshape(3, 29).astype(np.complex128), d)
+        assert _rel(y, ref) < _bound(29, double)
