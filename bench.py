@@ -45,6 +45,7 @@ import subprocess
 import sys
 import threading
 import time
+import traceback
 from pathlib import Path
 
 ROOT = Path(__file__).resolve().parent
@@ -1153,9 +1154,9 @@ def main():
 
     extras = {}
     if rank == 0 and world == 1 and args.workload == "configs" and not args.no_extras:
-        extras["batched_uneven"] = _extra(run_batched(args, rank, world, local_rank))
-        extras["serving"] = _extra(serving_in_child(args))
-        extras["precision_mode"] = run_precision(args, rank, world, local_rank)
+        extras["batched_uneven"] = _leg("batched_uneven", lambda: _extra(run_batched(args, rank, world, local_rank)))
+        extras["serving"] = _leg("serving", lambda: _extra(serving_in_child(args)))
+        extras["precision_mode"] = _leg("precision_mode", lambda: run_precision(args, rank, world, local_rank))
 
     if rank == 0:
         e2e_ms = res["e2e"]["ms_per_step"]
@@ -1217,8 +1218,21 @@ def serving_in_child(args) -> dict:
     window), as `python bench.py --workload serving` gives it."""
     cmd = [sys.executable, str(Path(__file__).resolve()), "--workload", "serving",
            "--serve-seconds", str(args.serve_seconds), "--serve-rate", str(args.serve_rate)]
-    out = subprocess.run(cmd, capture_output=True, text=True, check=True)
+    out = subprocess.run(cmd, stdout=subprocess.PIPE, text=True)  # (its messages go where this one's go)
+    if out.returncode != 0:
+        raise RuntimeError(f"the serving workload's process ended with status {out.returncode}")
     return json.loads(out.stdout.strip().splitlines()[-1])
+
+
+def _leg(name: str, run) -> dict:
+    """An extra key of the default line; one that fails is reported under its
+    key and does not take the finished measurements with it."""
+    try:
+        return run()
+    except Exception as e:  # noqa: BLE001
+        traceback.print_exc()
+        print(f"bench: the {name} leg failed: {e}", file=sys.stderr, flush=True)
+        return {"error": f"{type(e).__name__}: {e}"}
 
 
 def _extra(line: dict) -> dict:
