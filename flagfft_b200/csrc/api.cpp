@@ -41,6 +41,10 @@ struct PlanDesc {  // src/exec/c_api_internal.hpp:14-32
   int64_t smem_optin = 232448;
 };
 
+Transform transform_of(const PlanDesc &d) {
+  return d.real_forward ? Transform::R2C : d.real_inverse ? Transform::C2R : Transform::C2C;
+}
+
 struct Plan {
   PlanDesc desc;
   bool initialized = false;
@@ -165,7 +169,7 @@ flagfftResult build_plan(flagfftHandle *out, PlanDesc desc) {  // src/exec/c_api
     auto plan = std::make_unique<Plan>();
     plan->desc = desc;
     Planner planner(desc.is_double, desc.smem_optin);
-    const Transform tr = desc.real_forward ? Transform::R2C : desc.real_inverse ? Transform::C2R : Transform::C2C;
+    const Transform tr = transform_of(desc);
     if (is_2d) {
       const int64_t n0 = desc.n[0], n1 = desc.n[1];
       const int64_t h1 = n1 / 2 + 1;
@@ -225,6 +229,7 @@ flagfftResult exec_common(flagfftHandle h, const void *in, void *out, flagfftTyp
   if (has_dir && dir != FLAGFFT_FORWARD && dir != FLAGFFT_INVERSE) return FLAGFFT_INVALID_VALUE;
   std::lock_guard<std::mutex> lock(plan->mutex);
   if (plan->is_batch) {
+    if (!addressable(Transform::C2C, plan->desc.is_double, false, in, out)) return FLAGFFT_UNALIGNED_DATA;
     BatchProgram *bp = dir == FLAGFFT_INVERSE ? plan->binv.get() : plan->bfwd.get();
     cudaError_t e = cudaErrorInvalidValue;
     try {
@@ -244,6 +249,8 @@ flagfftResult exec_common(flagfftHandle h, const void *in, void *out, flagfftTyp
   }
   const Program *prog = pick(plan, in == out);
   if (prog == nullptr) return FLAGFFT_EXEC_FAILED;
+  if (!addressable(transform_of(plan->desc), plan->desc.is_double, prog->real_pairs, in, out))
+    return FLAGFFT_UNALIGNED_DATA;
   return run(plan, prog, in, out);
 }
 

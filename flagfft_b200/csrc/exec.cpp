@@ -1409,6 +1409,7 @@ std::unique_ptr<Program> lower_t(const NodePtr &root, Planner &planner, Transfor
       // A: z_j = x_2j + i x_2j+1 (j = j1 n2 + j2), FFT over j1, x W_L^{j2 k1} -> Y[j2][k1];
       // with an even row distance the pairs are the rows read as complex
       // elements, and the pass is a plain complex one (tile kernels apply)
+      prog->real_pairs = idist % 2 == 0;
       auto *pa = idist % 2 == 0
                      ? bld.add_pass(sa, IoKind::C2C, false, batch, n2, idist / 2, 1, n2, L, n1, 1, Buf::In,
                                     Buf::Scratch0, n1)
@@ -1435,6 +1436,7 @@ std::unique_ptr<Program> lower_t(const NodePtr &root, Planner &planner, Transfor
       bld.set_post_twiddle(pa->a, L);
       // B: inverse FFT over j2, z_j -> x_2j, x_2j+1 (j = k1 + n1 k2): with an
       // even row distance, complex elements of the output rows
+      prog->real_pairs = odist % 2 == 0;
       if (odist % 2 == 0)
         bld.add_pass(sb, IoKind::C2C, true, batch, n1, L, 1, n1, odist / 2, 1, n1, Buf::Scratch0, Buf::Out, n2);
       else
@@ -1450,6 +1452,7 @@ std::unique_ptr<Program> lower_t(const NodePtr &root, Planner &planner, Transfor
     // pre-processing into a workspace, then the complex transform into the
     // output rows reinterpreted as complex (C2R).
     if (batch > 65535) throw std::runtime_error("multi-pass batch above 65535");
+    prog->real_pairs = true;
     const RealTw<T> rtw = bld.table_rtw_split(n);
     if (t == Transform::R2C) {
       lower_c2c<T>(bld, *prog, core_node, false, L, batch, idist / 2, odist, Buf::In, Buf::Out);

@@ -50,10 +50,25 @@ struct Program {
   std::vector<std::unique_ptr<PassBase>> passes;
   std::vector<DevPtr> owned;  // tables and workspaces
   DevPtr scratch0, scratch1;
+  // The reals of a real transform are read or written as complex elements
+  // (the passes of a transform that does not fit one CTA): their buffer must
+  // start on a pair.
+  bool real_pairs = false;
   cudaError_t run(const void *in, void *out, cudaStream_t st) const;
   std::string describe() const;
   int launches() const;
 };
+
+// True when the kernels can address a call's buffers: complex elements on
+// boundaries of their size, reals on theirs, or on a pair's when real_pairs
+// (Program).  An address off them is a misaligned access on the device, so
+// every entry point asks first.
+inline bool addressable(Transform t, bool is_double, bool real_pairs, const void *in, const void *out) {
+  const size_t real = is_double ? 8 : 4, pair = 2 * real;
+  const size_t in_b = t == Transform::R2C && !real_pairs ? real : pair;
+  const size_t out_b = t == Transform::C2R && !real_pairs ? real : pair;
+  return reinterpret_cast<size_t>(in) % in_b == 0 && reinterpret_cast<size_t>(out) % out_b == 0;
+}
 
 // Layout of one batched 1-D or 2-D request in elements of its own types.
 struct Layout {

@@ -315,6 +315,7 @@ extern "C" flagfftResult flagfftB200PrecisionC2C(const flagfftComplex *idata, fl
   if (idata == nullptr || odata == nullptr || batch <= 0 || batch > (1 << 26)) return FLAGFFT_INVALID_VALUE;
   if (direction != FLAGFFT_FORWARD && direction != FLAGFFT_INVERSE) return FLAGFFT_INVALID_VALUE;
   if ((n != 256 && n != 4096) || (terms != 3 && terms != 6)) return FLAGFFT_NOT_SUPPORTED;
+  if (!addressable(Transform::C2C, false, false, idata, odata)) return FLAGFFT_UNALIGNED_DATA;
 #ifdef FFB_HOST_EMULATION
   (void)stream;
   return FLAGFFT_NOT_SUPPORTED;

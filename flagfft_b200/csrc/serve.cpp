@@ -44,6 +44,11 @@ double now_s() {
 }
 
 bool is_double_type(flagfftType t) { return t == FLAGFFT_Z2Z || t == FLAGFFT_D2Z || t == FLAGFFT_Z2D; }
+Transform transform_of(flagfftType t) {
+  return t == FLAGFFT_R2C || t == FLAGFFT_D2Z   ? Transform::R2C
+         : t == FLAGFFT_C2R || t == FLAGFFT_Z2D ? Transform::C2R
+                                                : Transform::C2C;
+}
 
 // Element sizes (bytes) of a type's input and output.
 void io_elems(flagfftType t, int64_t n, int64_t *in_b, int64_t *out_b) {
@@ -284,6 +289,7 @@ class Server {
       return FLAGFFT_SETUP_FAILED;
     }
     if (!tpl) return FLAGFFT_SETUP_FAILED;
+    if (!addressable(transform_of(type), is_double_type(type), tpl->prog->real_pairs, in, out)) return FLAGFFT_UNALIGNED_DATA;
     auto r = std::make_shared<Request>();
     r->type = type;
     r->n = n;
@@ -361,9 +367,7 @@ class Server {
     const bool dbl = is_double_type(type);
     auto pl = planners_.find(dbl);
     if (pl == planners_.end()) pl = planners_.emplace(dbl, std::make_unique<Planner>(dbl, 232448)).first;
-    const Transform tr = (type == FLAGFFT_R2C || type == FLAGFFT_D2Z)   ? Transform::R2C
-                         : (type == FLAGFFT_C2R || type == FLAGFFT_Z2D) ? Transform::C2R
-                                                                        : Transform::C2C;
+    const Transform tr = transform_of(type);
     NodePtr root = build_raw_root(*pl->second, n, nullptr, nullptr);
     if (!raw_supported(root)) return nullptr;
     Layout lay;

@@ -17,6 +17,12 @@
  * Data pointers are device pointers (in-place when idata == odata).  Exec is
  * asynchronous on the plan's stream (a cudaStream_t / CUstream, default the
  * legacy null stream).  The inverse transform is unnormalized.
+ *
+ * Complex data starts on a multiple of its element's size (8 or 16 bytes) and
+ * real data on a multiple of its own (4 or 8); the real data of a transform
+ * too long for one pass on a multiple of two elements, since its passes move
+ * pairs.  Exec answers FLAGFFT_UNALIGNED_DATA for other addresses, before any
+ * launch.
  */
 #ifndef FLAGFFT_H_
 #define FLAGFFT_H_
