@@ -1487,6 +1487,37 @@ std::unique_ptr<Program> lower_t(const NodePtr &root, Planner &planner, Transfor
   }
 }
 
+// The rows of a 2-D real transform whose row core does not fit one CTA or is
+// no core at all (a small factor times a prime above 19), as the 1-D real
+// lowering runs such lengths: `rows` rows of n reals and n / 2 + 1 bins,
+// through workspace 1 (the complex transform's own workspace is 0, which may
+// also be the buffer of the spectra: it holds them after or before that
+// transform).
+template <typename T>
+void lower_real_rows(Builder<T> &bld, Program &prog, const NodePtr &core, const NodePtr &full, bool inverse, int64_t n,
+                     int64_t rows, Buf src, Buf dst) {
+  if (rows > 65535) throw std::runtime_error("multi-pass 2-D real rows above 65535");
+  const int64_t L = n / 2, half = L + 1, width = n % 2 == 0 ? L : n;
+  ensure_scratch(prog.scratch1, (size_t)(rows * width) * sizeof(cpx<T>));
+  if (n % 2 == 0) {
+    prog.real_pairs = true;
+    const RealTw<T> rtw = bld.table_rtw_split(n);
+    if (!inverse) {
+      lower_c2c<T>(bld, prog, core, false, L, rows, L, L, src, Buf::Scratch1);
+      prog.passes.push_back(std::make_unique<RealPass<T>>(true, Buf::Scratch1, dst, rows, L, half, L, rtw));
+    } else {
+      prog.passes.push_back(std::make_unique<RealPass<T>>(false, src, Buf::Scratch1, rows, half, L, L, rtw));
+      lower_c2c<T>(bld, prog, core, true, L, rows, L, L, Buf::Scratch1, dst);
+    }
+    return;
+  }
+  prog.passes.push_back(std::make_unique<ConvertPass<T>>(inverse ? 2 : 0, src, Buf::Scratch1, rows,
+                                                         inverse ? half : n, n, n));
+  lower_c2c<T>(bld, prog, full, inverse, n, rows, n, n, Buf::Scratch1, Buf::Scratch1);
+  prog.passes.push_back(std::make_unique<ConvertPass<T>>(inverse ? 3 : 1, Buf::Scratch1, dst, rows, n,
+                                                         inverse ? n : half, n));
+}
+
 template <typename T>
 std::unique_ptr<Program> lower_2d_t(const NodePtr &root, Planner &planner, Transform t, bool inverse, int64_t n0,
                                     int64_t n1, int64_t batch) {
@@ -1513,23 +1544,25 @@ std::unique_ptr<Program> lower_2d_t(const NodePtr &root, Planner &planner, Trans
   }
   const bool even = (n1 % 2) == 0;
   NodePtr row_core = even ? build_raw_root(planner, n1 / 2, nullptr, nullptr) : root->row;
-  if (!bld.core_for(row_core, rs)) throw std::runtime_error("2-D real row axis too long for one CTA");
+  const bool row_onchip = bld.core_for(row_core, rs);
   const bool col_onchip = bld.core_for(root->col, cs);
   if (t == Transform::R2C) {
-    if (col_onchip) {
-      // rows into the workspace, then column tiles into the output (safe in place)
-      ensure_scratch(prog->scratch0, (size_t)(batch * n0 * h1) * sizeof(cpx<T>));
+    // rows into the workspace, then column tiles into the output (safe in
+    // place); for a column axis too long for one CTA rows into the output,
+    // transpose, the columns as rows (any lowering), transpose back
+    if (col_onchip) ensure_scratch(prog->scratch0, (size_t)(batch * n0 * h1) * sizeof(cpx<T>));
+    const Buf spectra = col_onchip ? Buf::Scratch0 : Buf::Out;
+    if (row_onchip) {
       auto *p = bld.add_pass(rs, even ? IoKind::R2C : IoKind::R2CFull, false, 1, batch * n0, 0, n1, even ? 2 : 1, 0,
-                             h1, 1, Buf::In, Buf::Scratch0, n1);
+                             h1, 1, Buf::In, spectra, n1);
       if (even) p->a.rtw = bld.table_rtw(n1);
+    } else {
+      lower_real_rows<T>(bld, *prog, row_core, root->row, false, n1, batch * n0, Buf::In, spectra);
+    }
+    if (col_onchip) {
       bld.add_pass(cs, IoKind::C2C, false, batch, h1, n0 * h1, 1, h1, n0 * h1, 1, h1, Buf::Scratch0, Buf::Out, n0);
       return prog;
     }
-    // a column axis too long for one CTA: rows into the output, transpose,
-    // the columns as rows (any lowering), transpose back
-    auto *p = bld.add_pass(rs, even ? IoKind::R2C : IoKind::R2CFull, false, 1, batch * n0, 0, n1, even ? 2 : 1, 0,
-                           h1, 1, Buf::In, Buf::Out, n1);
-    if (even) p->a.rtw = bld.table_rtw(n1);
     ensure_scratch(prog->scratch1, (size_t)(batch * n0 * h1) * sizeof(cpx<T>));
     prog->passes.push_back(std::make_unique<TransposePass<T>>(Buf::Out, Buf::Scratch1, batch, n0, h1));
     lower_c2c<T>(bld, *prog, root->col, false, n0, batch * h1, n0, n0, Buf::Scratch1, Buf::Scratch1);
@@ -1547,6 +1580,10 @@ std::unique_ptr<Program> lower_2d_t(const NodePtr &root, Planner &planner, Trans
     lower_c2c<T>(bld, *prog, root->col, true, n0, batch * h1, n0, n0, Buf::Scratch1, Buf::Scratch1);
     ensure_scratch(prog->scratch0, (size_t)(batch * n0 * h1) * sizeof(cpx<T>));
     prog->passes.push_back(std::make_unique<TransposePass<T>>(Buf::Scratch1, Buf::Scratch0, batch, h1, n0));
+  }
+  if (!row_onchip) {
+    lower_real_rows<T>(bld, *prog, row_core, root->row, true, n1, batch * n0, Buf::Scratch0, Buf::Out);
+    return prog;
   }
   auto *p = bld.add_pass(rs, even ? IoKind::C2R : IoKind::C2RFull, true, 1, batch * n0, 0, h1, 1, 0, n1, even ? 2 : 1,
                          Buf::Scratch0, Buf::Out, n1);

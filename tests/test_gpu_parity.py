@@ -267,3 +267,25 @@ def test_1701_row_forms(ffb, torch_cuda, batch, double, threads):
     for direction in (-1, 1):
         got = _run_c2c(ffb, torch_cuda, x, direction, double)
         _check(O.error_stats(got, O.c2c(x.astype(np.complex128), direction)), ftype, n)
+
+
+@pytest.mark.parametrize("double", [False, True], ids=["R2C_C2R", "D2Z_Z2D"])
+@pytest.mark.parametrize("n0,n1", [(64, 268), (33, 201), (512, 1359), (201, 1572)])
+def test_2d_real_rows_without_a_core(ffb, torch_cuda, n0, n1, double):
+    """2-D real transforms whose rows (or half rows) are a small factor times
+    a prime: the rows take the 1-D lowering of such lengths."""
+    torch = torch_cuda
+    fwd, inv = (ffb.D2Z, ffb.Z2D) if double else (ffb.R2C, ffb.C2R)
+    x = O.random_real(n0 * n1, n0 * n1, double).reshape(n0, n1)
+    a = torch.from_numpy(x).cuda()
+    y = torch.empty((n0, n1 // 2 + 1), dtype=torch.complex128 if double else torch.complex64, device="cuda")
+    z = torch.empty_like(a)
+    with ffb.plan2d(n0, n1, fwd) as p, ffb.plan2d(n0, n1, inv) as q:
+        p.execute(a, y)
+        ref = np.fft.rfft2(x.astype(np.float64))
+        assert O.error_stats(y.cpu().numpy().reshape(1, -1), ref.reshape(1, -1))["rel_l2"] <= \
+            O.north_star_bound(O.D2Z if double else O.R2C, n0 * n1)
+        q.execute(torch.from_numpy(ref.astype(y.cpu().numpy().dtype)).cuda(), z)
+        back = z.cpu().numpy().reshape(1, -1)
+        assert O.error_stats(back, x.astype(np.float64).reshape(1, -1) * (n0 * n1))["rel_l2"] <= \
+            O.north_star_bound(O.Z2D if double else O.C2R, n0 * n1)

@@ -272,3 +272,22 @@ def test_batch_convolution_rows_of_one_codelet(monkeypatch, double):
     for d, y in zip((-1, 1), outs):
         ref = O.c2c(O.random_complex(87, 5, double).reshape(3, 29).astype(np.complex128), d)
         assert _rel(y, ref) < _bound(29, double)
+
+
+# image rows whose half length (even) or length (odd) is a small factor times a
+# prime: 268 = 2 x 134 = 2 x (2 x 67), 201 = 3 x 67, 1359 = 9 x 151, 1572 = 2 x
+# 786 = 2 x (6 x 131); the column axis on chip, in two passes (201) and in a
+# convolution chain (20011)
+@pytest.mark.parametrize("n0,n1,double", [(16, 268, False), (5, 201, True), (32, 1359, False), (12, 1572, True),
+                                          (67, 219, False), (201, 268, True), (20011, 6, False), (201, 201, False)])
+def test_2d_real_rows_without_a_core(n0, n1, double):
+    x = O.random_real(n0 * n1, n0 + n1, True).reshape(n0, n1).astype(np.float64 if double else np.float32)
+    ref = np.fft.rfft2(x.astype(np.float64))
+    assert _rel(H.fft2(x, "r2c", double=double), ref) < _bound(n0 * n1, double)
+    assert _rel(H.fft2(ref, "c2r", n1, double), x.astype(np.float64) * n0 * n1) < _bound(n0 * n1, double)
+
+
+def test_2d_real_row_lengths_plan():
+    for n1 in range(32, 700):
+        H.lib().flagfftDestroy(H.plan2d(16, n1, R2C))
+        H.lib().flagfftDestroy(H.plan2d(16, n1, Z2D))
