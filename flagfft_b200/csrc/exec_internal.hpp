@@ -70,17 +70,17 @@ struct TilePass final : PassBase {
   }
 
   std::string describe() const override {
+    const TileKernel k = tile_kernel<T>(a, kind, io, smem);
     std::ostringstream o;
     o << (a.regcol ? "register-columns" : a.blue_pair ? "bluestein-four-step-pair" : a.blue_cols ? "bluestein-four-step" : kind_name(kind)) << "/" << io_name(io)
       << " "
       << (sizeof(T) == 4 ? "f32" : "f64") << " L=" << a.core.L
       << " radices=[";
     for (int s = 0; s < a.core.nst; ++s) o << (s ? "," : "") << a.core.radix[s];
-    o << "] n=" << a.n << " transforms=" << a.nbatch << "x" << a.G << " per_cta=" << a.W
-      << " threads=" << (a.blue_cols ? blue4_threads(a.blue_cols, a.core.L, a.blue_pair != 0) : a.mixed ? a.mixed : a.tiles ? a.tpt : a.W * a.tpt)
-      << (a.tiles ? " tiles" : a.mixed ? " mixed tiles" : "") << " smem=" << tile_smem<T>(a, kind, io, smem) << " " << buf_name(src) << "->"
+    o << "] n=" << a.n << " transforms=" << a.nbatch << "x" << a.G << " per_cta=" << k.W << " threads=" << k.threads
+      << k.name << (k.dense ? " 64-register" : "") << " smem=" << k.smem << " " << buf_name(src) << "->"
       << buf_name(dst);
-    if (a.tcols) o << " tma-columns(threads=" << a.tc_threads << " smem=" << a.tc_smem << ")";
+    if (k.columns) o << " " << k.columns << "(threads=" << k.col_threads << " smem=" << k.col_smem << ")";
     if (a.post_twiddle) o << " +twiddle";
     if (!note.empty()) o << " (" << note << ")";
     return o.str();

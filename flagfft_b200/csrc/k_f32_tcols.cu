@@ -16,6 +16,11 @@ bool tcols_eligible<float>(int L, long long nbatch, long long G, long long ib, l
 }
 
 template <>
+bool wide_columns<float>(const TileArgs<float> &a, int *threads, size_t *smem) {
+  return wcols::shape_any(a, threads, smem);
+}
+
+template <>
 long long tcols_wait_failures<float>() {
 #ifndef FFB_HOST_EMULATION
   int v = 0, w = 0;

@@ -15,6 +15,11 @@ bool tcols_eligible<double>(int L, long long nbatch, long long G, long long ib, 
 }
 
 template <>
+bool wide_columns<double>(const TileArgs<double> &, int *, size_t *) {
+  return false;
+}
+
+template <>
 long long tcols_wait_failures<double>() {
 #ifndef FFB_HOST_EMULATION
   int v = 0;

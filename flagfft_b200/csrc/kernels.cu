@@ -38,6 +38,8 @@ namespace rrows {
 // defined in k_*_rrows.cu
 template <typename T>
 cudaError_t launch(const TileArgs<T> &a, IoKind io, cudaStream_t s);
+template <typename T>
+bool shape(const TileArgs<T> &a, IoKind io, TileKernel *k);
 }  // namespace rrows
 
 namespace mixed {
@@ -436,21 +438,48 @@ cudaError_t launch_tile(const TileArgs<T> &a, CoreKind kind, IoKind io, size_t s
 }
 
 template <typename T>
-size_t tile_smem(const TileArgs<T> &a, CoreKind kind, IoKind io, size_t smem) {
+TileKernel tile_kernel(const TileArgs<T> &a, CoreKind kind, IoKind io, size_t smem) {
   const int k = (int)kind;
-  if (a.regcol) return 0;
-  if (a.blue_cols) return blue4_smem(a.blue_cols, a.core.L, sizeof(cpx<T>), a.blue_pair != 0);
-  if (a.tiles || a.mixed) return smem;
-  if (a.pp && io == IoKind::C2C && (k == 0 || k == 1 || k == 3)) {
+  TileKernel t;
+  t.W = a.W;
+  t.threads = a.W * a.tpt;
+  t.smem = smem;
+  if (a.regcol) {
+    t.smem = 0;
+    return t;
+  }
+  if (a.blue_cols) {
+    t.threads = blue4_threads(a.blue_cols, a.core.L, a.blue_pair != 0);
+    t.smem = blue4_smem(a.blue_cols, a.core.L, sizeof(cpx<T>), a.blue_pair != 0);
+    return t;
+  }
+  if (a.tcols) {
+    const bool wide = wide_columns<T>(a, &t.col_threads, &t.col_smem);
+    t.columns = wide ? "wide-tma-columns" : "tma-columns";
+    if (!wide) {
+      t.col_threads = a.tc_threads;
+      t.col_smem = (size_t)a.tc_smem;
+    }
+  }
+  if (a.tiles) {
+    t.name = " tiles";
+    t.threads = a.tpt;
+  } else if (k == 0 && (io == IoKind::R2C || io == IoKind::C2R) && rrows::shape<T>(a, io, &t)) {
+    t.name = " real rows";
+  } else if (a.mixed) {
+    t.name = " mixed tiles";
+    t.threads = a.mixed;
+  } else if (a.pp && io == IoKind::C2C && (k == 0 || k == 1 || k == 3)) {
     const size_t r = k == 0 ? rows::rows_smem_any<T, 0>(a) : k == 1 ? rows::rows_smem_any<T, 1>(a)
                                                                      : rows::rows_smem_any<T, 3>(a);
-    if (r) return r;
+    if (r) t.smem = r;
+    t.dense = k == 0 ? rows::rows_dense_any<T, 0>(a) : k == 1 && rows::rows_dense_any<T, 1>(a);
   }
-  return smem;
+  return t;
 }
 
-template size_t tile_smem<float>(const TileArgs<float> &, CoreKind, IoKind, size_t);
-template size_t tile_smem<double>(const TileArgs<double> &, CoreKind, IoKind, size_t);
+template TileKernel tile_kernel<float>(const TileArgs<float> &, CoreKind, IoKind, size_t);
+template TileKernel tile_kernel<double>(const TileArgs<double> &, CoreKind, IoKind, size_t);
 template cudaError_t launch_tile<float>(const TileArgs<float> &, CoreKind, IoKind, size_t, cudaStream_t);
 template cudaError_t launch_tile<double>(const TileArgs<double> &, CoreKind, IoKind, size_t, cudaStream_t);
 

@@ -233,10 +233,21 @@ cudaError_t launch_real_pre(const cpx<T> *x, cpx<T> *z, long long batch, long lo
 
 template <typename T>
 cudaError_t launch_tile(const TileArgs<T> &a, CoreKind kind, IoKind io, size_t smem_bytes, cudaStream_t stream);
-// Dynamic shared memory the launch of a tile pass uses (the row kernels of
-// the compile-time sequences take less than the pass's general figure).
+// The kernel launch_tile takes for a pass whose buffers keep its copy rules:
+// transforms and threads per CTA and dynamic shared memory.  columns (a TMA
+// column kernel; null: none) then runs in its place, with col_threads and
+// col_smem, and the rest describes the fallback for other buffers.
+struct TileKernel {
+  const char *name = "";  // tiles, mixed tiles, real rows; empty: rows, ping-pong or in-place tiles by the pass
+  int W = 0, threads = 0;
+  size_t smem = 0;
+  bool dense = false;  // the 64-register row kernels
+  const char *columns = nullptr;
+  int col_threads = 0;
+  size_t col_smem = 0;
+};
 template <typename T>
-size_t tile_smem(const TileArgs<T> &a, CoreKind kind, IoKind io, size_t smem_bytes);
+TileKernel tile_kernel(const TileArgs<T> &a, CoreKind kind, IoKind io, size_t smem_bytes);
 
 // Strided tile kernels of the compile-time sequences (TileArgs::tiles);
 // defined in k_f32_tiles.cu / k_f64_tiles.cu.  tiles_shape gives the tile
@@ -257,6 +268,9 @@ cudaError_t launch_tcols(const TileArgs<T> &a, cudaStream_t stream);
 template <typename T>
 bool tcols_eligible(int L, long long nbatch, long long G, long long ib, long long ig, long long ii, long long ob,
                     long long og, long long ok, int *threads, size_t *smem);
+// wide_columns: the pass runs on the wide column kernel (wcols.cuh).
+template <typename T>
+bool wide_columns(const TileArgs<T> &a, int *threads, size_t *smem);
 template <typename T>
 long long tcols_wait_failures();
 

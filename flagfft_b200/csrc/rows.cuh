@@ -552,6 +552,26 @@ size_t rows_smem(const TileArgs<T> &a) {
   return (size_t)a.W * slot_len<L>() * sizeof(cpx<T>);
 }
 
+// Single-precision passes of many rows: a form of 64 registers, two 512-thread
+// CTAs' worth of rows per SM instead of one, without spills to speak of.  Its
+// rows each take longer (less of a butterfly's latency is hidden within a
+// thread), so it is for passes whose rows come in several waves: kDensePoints
+// points or more.  Measured (us, 96-128 registers -> 64): C2C 4096 x 4096 56.2
+// -> 49.1, 8192 x 2048 80.2 -> 64.5, Bluestein 4079 x 2000 139 -> 119, 2039 x
+// 4000 94.9 -> 87.6, 509 x 20000 94.8 -> 87.6; but 4096 x 256 5.7 -> 7.0, 8192 x
+// 100 6.0 -> 8.4, 1009 x 1024 12.9 -> 14.5, 509 x 2000 12.1 -> 13.8.  Plain
+// rows of 2048 points or fewer move HBM at its rate either way (1024 x 16384
+// 44.7 -> 44.4), and 1536 loses (8000 rows 36.3 -> 42.1).
+constexpr long long kDensePoints = 1ll << 22;
+template <typename T, int KIND, int L>
+constexpr bool rows_dense() {
+  return sizeof(T) == 4 && (L & (L - 1)) == 0 && L <= 8192 && (KIND == 0 ? L >= 4096 : KIND == 1 && L >= 1024);
+}
+template <typename T, int KIND, int L>
+bool rows_run_dense(const TileArgs<T> &a) {
+  return rows_dense<T, KIND, L>() && a.nbatch * a.G * (long long)L >= kDensePoints;
+}
+
 #ifndef FFB_HOST_EMULATION
 template <typename T, int KIND, bool INV, int MB, int L, int TPT, int... Rs>
 cudaError_t launch_rows_mb(const TileArgs<T> &a, cudaStream_t s) {
@@ -572,25 +592,10 @@ template <typename T, int KIND, int L>
 constexpr int rows_min_blocks() {
   return sizeof(T) == 8 && KIND == 0 && L <= 4096 ? 2 : 1;
 }
-// Single-precision passes of many rows: a form of 64 registers, two 512-thread
-// CTAs' worth of rows per SM instead of one, without spills to speak of.  Its
-// rows each take longer (less of a butterfly's latency is hidden within a
-// thread), so it is for passes whose rows come in several waves: kDensePoints
-// points or more.  Measured (us, 96-128 registers -> 64): C2C 4096 x 4096 56.2
-// -> 49.1, 8192 x 2048 80.2 -> 64.5, Bluestein 4079 x 2000 139 -> 119, 2039 x
-// 4000 94.9 -> 87.6, 509 x 20000 94.8 -> 87.6; but 4096 x 256 5.7 -> 7.0, 8192 x
-// 100 6.0 -> 8.4, 1009 x 1024 12.9 -> 14.5, 509 x 2000 12.1 -> 13.8.  Plain
-// rows of 2048 points or fewer move HBM at its rate either way (1024 x 16384
-// 44.7 -> 44.4), and 1536 loses (8000 rows 36.3 -> 42.1).
-constexpr long long kDensePoints = 1ll << 22;
-template <typename T, int KIND, int L>
-constexpr bool rows_dense() {
-  return sizeof(T) == 4 && (L & (L - 1)) == 0 && L <= 8192 && (KIND == 0 ? L >= 4096 : KIND == 1 && L >= 1024);
-}
 template <typename T, int KIND, bool INV, int L, int TPT, int... Rs>
 cudaError_t launch_rows(const TileArgs<T> &a, cudaStream_t s) {
   if constexpr (rows_dense<T, KIND, L>()) {
-    if (a.nbatch * a.G * (long long)L >= kDensePoints) return launch_rows_mb<T, KIND, INV, 2, L, TPT, Rs...>(a, s);
+    if (rows_run_dense<T, KIND, L>(a)) return launch_rows_mb<T, KIND, INV, 2, L, TPT, Rs...>(a, s);
   }
   return launch_rows_mb<T, KIND, INV, rows_min_blocks<T, KIND, L>(), L, TPT, Rs...>(a, s);
 }
@@ -620,6 +625,18 @@ size_t rows_smem_any(const TileArgs<T> &a) {
   FFB_FIXED_SEQUENCES(FFB_ROWS_SMEM)
 #undef FFB_ROWS_SMEM
   return 0;
+}
+
+// The row kernel that runs the pass is the 64-register form.
+template <typename T, int KIND>
+bool rows_dense_any(const TileArgs<T> &a) {
+#define FFB_ROWS_DENSE(L, ...)                                                                \
+  if (rows_fit<T, KIND, L, rows_tpt<T, L, __VA_ARGS__>(), __VA_ARGS__>(a) ||                 \
+      rows_fit<T, KIND, L, rows_tpt_wide<T, L, __VA_ARGS__>(), __VA_ARGS__>(a))              \
+    return rows_run_dense<T, KIND, L>(a);
+  FFB_FIXED_SEQUENCES(FFB_ROWS_DENSE)
+#undef FFB_ROWS_DENSE
+  return false;
 }
 
 // Launches the row kernel of the pass's sequence; cudaErrorNotSupported when

@@ -129,6 +129,29 @@ __global__ void __launch_bounds__(tile::TileBounds<T>::kMaxThreads, MB)
                                           reinterpret_cast<cpx<T> *>(smraw), rows::DevT{});
 }
 
+// Rows per CTA: the executor's rule for row passes (about 128 threads, no more
+// than keeps two CTAs per SM busy); 0 when no CTA holds a row.
+template <typename T, int L>
+long long rows_per_cta(const TileArgs<T> &a, int tpt) {
+  const size_t per = slot_len<L>() * sizeof(cpx<T>);
+  if (per > 232448) return 0;
+  return std::max<long long>(
+      1, std::min<long long>({128 / tpt, (long long)(110 * 1024 / per), a.nbatch * a.G / (2 * 148), (long long)a.G}));
+}
+
+// Many rows: the 64-register form (rows.cuh rows_dense says when and why).
+// Measured (us, R2C / C2R): 2048 x 8192 31.0 / 35.1 -> 29.5 / 32.8, 8192 x 1024
+// 18.5 / 24.6 -> 17.3 / 19.1, 16384 x 512 27.1 / 31.4 -> 22.5 / 25.7; 1024 x 64
+// 4.2 / 4.6 -> 6.2 / 6.3, 3072 x 2000 14.2 / 14.5 -> 17.9 / 16.9
+template <typename T, int L>
+constexpr bool has_dense() {
+  return sizeof(T) == 4 && (L & (L - 1)) == 0 && L >= 512 && L <= 8192;
+}
+template <typename T, int L>
+bool run_dense(const TileArgs<T> &a) {
+  return has_dense<T, L>() && a.nbatch * a.G * (long long)L >= rows::kDensePoints;
+}
+
 template <typename T, bool INV, int L, int... Rs>
 cudaError_t launch_seq(const TileArgs<T> &a, cudaStream_t s) {
   if constexpr (slot_len<L>() * sizeof(cpx<T>) > 232448) {  // (no CTA holds such a row)
@@ -137,21 +160,13 @@ cudaError_t launch_seq(const TileArgs<T> &a, cudaStream_t s) {
     return cudaErrorNotSupported;
   } else {
   constexpr int TPT = rows::rows_tpt<T, L, Rs...>();
-  // rows per CTA: the executor's rule for row passes (about 128 threads, no
-  // more than keeps two CTAs per SM busy)
   const size_t per = slot_len<L>() * sizeof(cpx<T>);
-  const long long W = std::max<long long>(
-      1, std::min<long long>({128 / TPT, (long long)(110 * 1024 / per), a.nbatch * a.G / (2 * 148), (long long)a.G}));
+  const long long W = rows_per_cta<T, L>(a, TPT);
   const long long tiles = (a.G + W - 1) / W;
 #ifndef FFB_HOST_EMULATION
   const dim3 grid((unsigned)tiles, (unsigned)a.nbatch), block((unsigned)(W * TPT));
-  // many rows: the 64-register form (rows.cuh rows_dense says when and why).
-  // Measured (us, R2C / C2R): 2048 x 8192 31.0 / 35.1 -> 29.5 / 32.8, 8192 x 1024
-  // 18.5 / 24.6 -> 17.3 / 19.1, 16384 x 512 27.1 / 31.4 -> 22.5 / 25.7; 1024 x 64
-  // 4.2 / 4.6 -> 6.2 / 6.3, 3072 x 2000 14.2 / 14.5 -> 17.9 / 16.9
-  constexpr bool dense = sizeof(T) == 4 && (L & (L - 1)) == 0 && L >= 512 && L <= 8192;
-  if constexpr (dense) {
-    if (a.nbatch * a.G * (long long)L >= rows::kDensePoints) {
+  if constexpr (has_dense<T, L>()) {
+    if (run_dense<T, L>(a)) {
       cudaError_t e = set_smem_limit_once<k_rrows<T, INV, 2, L, TPT, Rs...>>(232448);
       if (e != cudaSuccess) return e;
       return launch_pdl(k_rrows<T, INV, 2, L, TPT, Rs...>, grid, block, (size_t)W * per, s, a, (int)W);
@@ -175,6 +190,35 @@ cudaError_t launch_seq(const TileArgs<T> &a, cudaStream_t s) {
   }
 }
 
+// Half-length real rows whose distances keep every row on a pair (the base
+// address is checked at launch).
+template <typename T>
+bool layout_fits(const TileArgs<T> &a, IoKind io) {
+  const bool inv = io == IoKind::C2R;
+  const long long dist = inv ? a.og : a.ig, bdist = inv ? a.ob : a.ib;
+  return dist % 2 == 0 && (a.nbatch <= 1 || bdist % 2 == 0) && (inv ? a.ii : a.ok) == 1 && (inv ? a.ok : a.ii) == 2 &&
+         a.nbatch <= 65535;
+}
+
+// Shape of the row kernel that runs the pass (rows and threads per CTA, shared
+// memory, the 64-register form); false when none does.
+template <typename T>
+bool shape(const TileArgs<T> &a, IoKind io, TileKernel *k) {
+  if (!layout_fits(a, io)) return false;
+#define FFB_RROWS_SHAPE(L, ...)                                                \
+  if (tile::core_is<L, __VA_ARGS__>(a.core)) {                                 \
+    const int tpt = rows::rows_tpt<T, L, __VA_ARGS__>();                       \
+    k->W = (int)rows_per_cta<T, L>(a, tpt);                                    \
+    k->threads = k->W * tpt;                                                   \
+    k->smem = (size_t)k->W * slot_len<L>() * sizeof(cpx<T>);                   \
+    k->dense = run_dense<T, L>(a);                                             \
+    return k->W > 0;                                                           \
+  }
+  FFB_FIXED_SEQUENCES(FFB_RROWS_SHAPE)
+#undef FFB_RROWS_SHAPE
+  return false;
+}
+
 // Launches a half-length real pass (IoKind R2C or C2R of a Dit core) on the
 // row kernel of its core's sequence; cudaErrorNotSupported when the core is
 // not one, or a row of reals does not start on a pair (the mixed-radix or the
@@ -182,11 +226,8 @@ cudaError_t launch_seq(const TileArgs<T> &a, cudaStream_t s) {
 template <typename T>
 cudaError_t launch(const TileArgs<T> &a, IoKind io, cudaStream_t s) {
   const bool inv = io == IoKind::C2R;
-  const long long dist = inv ? a.og : a.ig, bdist = inv ? a.ob : a.ib;
-  const void *base = inv ? a.out : a.in;
-  if (reinterpret_cast<uintptr_t>(base) % sizeof(cpx<T>) != 0 || dist % 2 != 0 || (a.nbatch > 1 && bdist % 2 != 0))
+  if (reinterpret_cast<uintptr_t>(inv ? a.out : a.in) % sizeof(cpx<T>) != 0 || !layout_fits(a, io))
     return cudaErrorNotSupported;
-  if ((inv ? a.ii : a.ok) != 1 || (inv ? a.ok : a.ii) != 2 || a.nbatch > 65535) return cudaErrorNotSupported;
 #define FFB_RROWS_TRY(L, ...)                \
   if (tile::core_is<L, __VA_ARGS__>(a.core)) \
     return inv ? launch_seq<T, true, L, __VA_ARGS__>(a, s) : launch_seq<T, false, L, __VA_ARGS__>(a, s);

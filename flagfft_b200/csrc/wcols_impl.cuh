@@ -110,6 +110,26 @@ cudaError_t launch_seq(const TileArgs<float> &a, cudaStream_t) {
 
 #endif
 
+// Threads and shared memory of the kernel for a pass whose buffers keep the
+// copy rules; false when the column kernel takes it.
+inline bool shape_any(const TileArgs<float> &a, int *threads, size_t *smem) {
+  if (a.chirp_mode != 0 || a.nbatch <= 0) return false;
+  alignas(16) static unsigned char probe[16];
+  TileArgs<float> b = a;
+  b.in = b.out = probe;
+  Args p{};
+  bool out_rows = false;
+#define FFB_WCOLS_SHAPE(L, ...)                      \
+  if (tile::core_is<L, __VA_ARGS__>(a.core)) {       \
+    *threads = Shape<L, __VA_ARGS__>::NT;            \
+    *smem = Shape<L, __VA_ARGS__>::smem;             \
+    return make_args<L, Shape<L, __VA_ARGS__>>(b, &p, &out_rows); \
+  }
+  FFB_TCOLS_SEQUENCES(FFB_WCOLS_SHAPE)
+#undef FFB_WCOLS_SHAPE
+  return false;
+}
+
 // cudaErrorNotSupported: the column kernel takes the pass.
 inline cudaError_t launch_any(const TileArgs<float> &a, cudaStream_t s) {
   if (a.chirp_mode != 0 || a.nbatch <= 0) return cudaErrorNotSupported;
