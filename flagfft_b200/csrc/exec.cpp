@@ -565,7 +565,8 @@ class Builder {
   // Radix chain of the pass on the mixed-radix tile kernel (mixed.cuh), or
   // empty when another kernel takes it: a compile-time row, tile or TMA
   // column sequence, a pass of a batch program (whose persistent kernel runs
-  // the ping-pong body), a single codelet, a layout the kernel does not read,
+  // the body on the pass's own chain), a single codelet, a layout the kernel
+  // does not read,
   // or two buffers too long for one CTA.  The first and last stage move runs
   // of L/R0 and L/R_last elements of global memory, so both are kept at four
   // (32 bytes in single precision) or more.
@@ -583,10 +584,12 @@ class Builder {
       int tw = 0, th = 0;
       size_t sm = 0;
       if (fixed && spec.kind == CoreKind::Dit && strided) {
-        // (the column kernel's own sequence: it declines at launch when its
-        // tiles are too few, or its buffers break the copy rules)
-        if (tcols(spec, io, nbatch, G, ib, ig, ii, ob, og, ok, &th, &sm))
-          return nbatch <= 65535 && mixed_fits(spec, io, seq, 4) ? seq : std::vector<int>{};
+        // The column kernel keeps every pass that it can copy (buffers off
+        // its rules take the tile kernel).  Against it the narrow tiles were
+        // slower however few its groups: columns of a 2-D C2C, us here and
+        // there with the rows, 1024 x 16 14.2 / 10.6, x 128 13.2 / 8.8, x 512
+        // 15.8 / 12.4, 2048 x 128 11.7 / 9.7; Z2Z 1536 x 16 12.0 / 10.9.
+        if (tcols(spec, io, nbatch, G, ib, ig, ii, ob, og, ok, &th, &sm)) return {};
         // (a tile kernel with fewer CTAs than SMs leaves some idle)
         if (tiles_shape<T>((int)L, &tw, &th, &sm) && nbatch * (G / tw) >= kSMs) return {};
       }
@@ -598,21 +601,21 @@ class Builder {
     // (a half-length real pass of a compile-time sequence keeps it: the real
     // row kernel takes it whenever its rows start on pairs)
     if (fixed && spec.kind == CoreKind::Dit && (io == IoKind::R2C || io == IoKind::C2R))
-      return mixed_fits(spec, io, seq, 1) ? seq : std::vector<int>{};
+      return mixed_fits(spec, io, seq) ? seq : std::vector<int>{};
     std::vector<int> r;
     if (!mixed_chain(L, 0, &r) && !mixed_chain(L, 1, &r)) return {};
-    return mixed_fits(spec, io, r, 1) ? r : std::vector<int>{};
+    return mixed_fits(spec, io, r) ? r : std::vector<int>{};
   }
 
-  // W transforms of the chain fit one CTA and its global runs are long enough.
-  static bool mixed_fits(const CoreSpec &spec, IoKind io, const std::vector<int> &r, int W) {
+  // A transform of the chain fits one CTA and its global runs are long enough.
+  static bool mixed_fits(const CoreSpec &spec, IoKind io, const std::vector<int> &r) {
     const int64_t L = spec.L;
     if (r.size() < 2 || (int)r.size() > kMaxStages || L / r.front() < 4 || L / r.back() < 4) return false;
     Core c{};
     c.L = (int)L;
     c.nst = (int)r.size();
     c.radix[0] = r[0];
-    return (size_t)W * ((size_t)mixed::slot_len(c, mixed::buffers(c, spec.kind, io)) + 2) * sizeof(cpx<T>) <= 232448;
+    return ((size_t)mixed::slot_len(c, mixed::buffers(c, spec.kind, io)) + 2) * sizeof(cpx<T>) <= 232448;
   }
 
   // The column kernel takes the pass (tcols.cuh).
@@ -780,15 +783,6 @@ class Builder {
       if (W_overflows(a.W, L, ig, ii) || W_overflows(a.W, L, og, ok))
         throw std::runtime_error("tile extent above 2^31 elements");
       a.tpt = 1;
-      {
-        int th = 0;
-        size_t sm = 0;
-        if (tcols(spec, io, nbatch, G, ib, ig, ii, ob, og, ok, &th, &sm)) {
-          a.tcols = 1;
-          a.tc_threads = th;
-          a.tc_smem = (int)sm;
-        }
-      }
       a.wdiv = make_fastdiv((uint32_t)a.W);
       a.pairs_div = make_fastdiv((uint32_t)(std::max<int64_t>(0, logical_n) / 2 / 2 + 1));
       p->kind = spec.kind;

@@ -124,19 +124,11 @@ inline int sm_count() {
   return n > 0 ? n : 148;
 }
 
-// Groups below which a pass leaves too many SMs idle here, and the mixed-radix
-// kernel's narrower tiles take it where the pass has them (TileArgs::mixed).
-// Measured (us, here -> mixed-radix tiles): 64 groups (C2C 2^19 x 1, with its
-// 512-point pass) 20.0 -> 18.8, (Z2Z 2^19 x 1) 25.9 -> 20.0; 128 groups (C2C
-// 2^20 x 1) 16.5 -> 25.1, (2-D 1024 x 1024) 13.6 -> 18.6.
-constexpr long long kMinGroups = 96;
-
 template <typename T, bool INV, int L, int... Rs>
 cudaError_t launch_seq(const TileArgs<T> &a, cudaStream_t s) {
   using Sh = Shape<T, L, Rs...>;
   Args<T> p{};
   if (!make_views<T, L, Sh::GC, Sh::RB>(a, &p)) return cudaErrorNotSupported;
-  if (a.mixed && p.total_groups < kMinGroups) return cudaErrorNotSupported;
   if (!encode<T>(p.in_view, &p.in_map) || !encode<T>(p.out_view, &p.out_map)) return cudaErrorNotSupported;
   const long long ctas = std::min<long long>(p.total_groups, sm_count());
   cudaError_t e;

@@ -1,0 +1,52 @@
+"""Which kernel takes a strided pass of a compile-time sequence: the column
+kernel wherever it can copy the pass, the tile kernel from one CTA per SM on,
+the mixed-radix tiles below.  Host-emulation build (the rules are the plan's)."""
+import ctypes
+
+import numpy as np
+import pytest
+
+import hostcheck as H
+
+C2C, Z2Z = 0x29, 0x69
+
+
+def _column_pass(n0, n1, code):
+    plan = H.plan2d(n0, n1, code)
+    text = H.describe(plan).split("-- Forward execution --")[-1].split("-- Inverse execution --")[0]
+    H.lib().flagfftDestroy(plan)
+    return [ln for ln in text.splitlines() if ln.strip().startswith("pass ")][1]
+
+
+@pytest.mark.parametrize("n0,n1,code", [(1024, 16, C2C), (1024, 256, C2C), (1536, 24, C2C), (2048, 128, C2C),
+                                        (1024, 64, Z2Z), (1536, 16, Z2Z), (2048, 8, Z2Z)])
+def test_column_kernel_keeps_few_groups(n0, n1, code):
+    line = _column_pass(n0, n1, code)
+    assert "tma-columns(" in line and "mixed tiles" not in line, line
+
+
+@pytest.mark.parametrize("n0,n1,code", [(512, 256, C2C), (256, 512, C2C), (256, 512, Z2Z), (512, 512, Z2Z)])
+def test_narrow_tiles_below_one_cta_per_sm(n0, n1, code):
+    assert "mixed tiles" in _column_pass(n0, n1, code)
+
+
+@pytest.mark.parametrize("n0,n1,code", [(256, 2376, C2C), (512, 2400, C2C), (256, 2376, Z2Z)])
+def test_tile_kernel_from_one_cta_per_sm(n0, n1, code):
+    line = _column_pass(n0, n1, code)
+    assert " tiles smem" in line and "mixed" not in line and "tma-columns" not in line, line
+
+
+@pytest.mark.parametrize("n0,n1", [(1024, 20), (2048, 24)])
+def test_columns_off_16_bytes(n0, n1):
+    """Single-precision columns of a buffer on 8 bytes only: the tile kernel."""
+    rng = np.random.default_rng(n0)
+    raw = (rng.uniform(-1, 1, n0 * n1 + 4) + 1j * rng.uniform(-1, 1, n0 * n1 + 4)).astype(np.complex64)
+    first = 1 if raw.ctypes.data % 16 == 0 else 0
+    x = raw[first:first + n0 * n1]
+    assert x.ctypes.data % 16 == 8
+    out = np.empty_like(raw)[first:first + n0 * n1]
+    plan = H.plan2d(n0, n1, C2C)
+    assert H.lib().flagfftExecC2C(plan, ctypes.c_void_p(x.ctypes.data), ctypes.c_void_p(out.ctypes.data), -1) == 0
+    H.lib().flagfftDestroy(plan)
+    ref = np.fft.fft2(x.reshape(n0, n1).astype(np.complex128)).ravel()
+    assert np.linalg.norm(out - ref) <= 5e-7 * np.log2(n0 * n1) * np.linalg.norm(ref)
