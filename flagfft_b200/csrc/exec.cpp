@@ -590,8 +590,14 @@ class Builder {
         // there with the rows, 1024 x 16 14.2 / 10.6, x 128 13.2 / 8.8, x 512
         // 15.8 / 12.4, 2048 x 128 11.7 / 9.7; Z2Z 1536 x 16 12.0 / 10.9.
         if (tcols(spec, io, nbatch, G, ib, ig, ii, ob, og, ok, &th, &sm)) return {};
-        // (a tile kernel with fewer CTAs than SMs leaves some idle)
-        if (tiles_shape<T>((int)L, &tw, &th, &sm) && nbatch * (G / tw) >= kSMs) return {};
+        // A tile kernel with fewer CTAs than SMs leaves some idle.  In single
+        // precision a sequence with radices other than 2^k gains from the
+        // narrow tiles only where it would leave half of them idle
+        // (1701-point columns, us here and there with the rows: x 192 19.2 /
+        // 22.0, x 512 22.9 / 22.4, x 1024 24.4 / 23.3 and, off 16 bytes, 29.7 /
+        // 24.8).
+        const int64_t enough = sizeof(T) == 4 && (L & (L - 1)) != 0 ? kSMs / 2 : kSMs;
+        if (tiles_shape<T>((int)L, &tw, &th, &sm) && nbatch * (G / tw) >= enough) return {};
       }
     } else if (io == IoKind::R2C ? (ii != 2 || ok != 1) : io == IoKind::C2R ? (ii != 1 || ok != 2)
                : io == IoKind::R2CFull || io == IoKind::C2RFull ? (ii != 1 || ok != 1) : true) {
@@ -662,14 +668,22 @@ class Builder {
   static size_t choose_mixed(TileArgs<T> &a, CoreKind kind, IoKind io, bool strided) {
     const int regs = sizeof(T) == 4 ? (a.mixed_set == 0 ? 80 : 128) : (a.mixed_set == 0 ? 128 : 255);
     const int64_t most = std::min<int64_t>(a.G, 64);
-    // strided tiles move 64 bytes of a row, or 32 where that would leave SMs
-    // without a tile
+    // Strided tiles move 64 bytes of a row, or 32 where that would leave SMs
+    // without a tile; in single precision only for three stages or more (two
+    // leave a narrow tile a warp or two of butterflies).  Measured (us, 64
+    // bytes / 32): 256 points (16 16) C2C 65536 x 4 11.4 / 13.1, R2C 131072 x 4
+    // 17.5 / 21.0, 2-D 256 x 64 8.0 / 10.9, 240 (16 15) x 1024 10.1 / 12.1, but
+    // 180 (15 12) x 1024 7.8 / 7.4; three stages 512 (8 8 8) C2C 2^18 x 2 20.9
+    // / 13.3, 2-D 300 x 128 7.9 / 6.9; double precision 256 (8 8 4) Z2Z 2-D
+    // 256 x 512 9.5 / 8.8.
     int64_t least = 1;
     const int64_t wide = sizeof(T) == 4 ? 8 : 4;
-    if (strided)
-      for (least = std::min<int64_t>(a.nbatch * a.G / wide < kSMs ? wide / 2 : wide, a.G);
+    if (strided) {
+      const bool halve = a.nbatch * a.G / wide < kSMs && (sizeof(T) == 8 || a.core.nst > 2);
+      for (least = std::min<int64_t>(halve ? wide / 2 : wide, a.G);
            least > 1 && mixed::smem_bytes(a, kind, io, (int)least) > 232448; --least) {
       }
+    }
     double best = 1e300;
     for (int NT = 64; NT <= mixed::kMaxThreads; NT += 32)
       for (int64_t W = least; W <= most; ++W) {

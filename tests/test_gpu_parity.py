@@ -289,3 +289,29 @@ def test_2d_real_rows_without_a_core(ffb, torch_cuda, n0, n1, double):
         back = z.cpu().numpy().reshape(1, -1)
         assert O.error_stats(back, x.astype(np.float64).reshape(1, -1) * (n0 * n1))["rel_l2"] <= \
             O.north_star_bound(O.Z2D if double else O.C2R, n0 * n1)
+
+
+# (n0, n1, double, the column pass's kernel in the description): passes above
+# the line each kernel starts at, with a part tile or group at the end
+@pytest.mark.parametrize("n0,n1,double,kernel", [
+    (256, 2376, False, " tiles smem"), (512, 2376, False, " tiles smem"), (1701, 594, False, " tiles smem"),
+    (256, 2376, True, " tiles smem"), (512, 2376, True, " tiles smem"), (1701, 2376, True, " tiles smem"),
+    (1024, 50, False, " tma-columns("), (2048, 770, False, " tma-columns("), (1024, 403, True, " tma-columns("),
+    (2048, 203, True, " tma-columns("), (256, 198, False, " mixed tiles "), (512, 301, True, " mixed tiles ")])
+def test_2d_columns_by_kernel(ffb, torch_cuda, n0, n1, double, kernel):
+    torch = torch_cuda
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(n0 + n1)
+    real = torch.float64 if double else torch.float32
+    x = torch.view_as_complex(torch.randn(n0, n1, 2, generator=gen, device="cuda", dtype=real))
+    y = torch.empty_like(x)
+    with ffb.plan2d(n0, n1, ffb.Z2Z if double else ffb.C2C) as p:
+        columns = [ln for ln in p.description().splitlines() if ln.strip().startswith("pass 1:")][0]
+        assert f"L={n0} " in columns and kernel in columns and "wide" not in columns, columns
+        assert ("mixed tiles" in columns) == (kernel == " mixed tiles ") and \
+            ("tma-columns" in columns) == (kernel == " tma-columns("), columns
+        for d, f in ((ffb.FORWARD, np.fft.fft2), (ffb.INVERSE, lambda v: np.fft.ifft2(v, norm="forward"))):
+            p.execute(x, y, d)
+            ref = f(x.cpu().numpy().astype(np.complex128))
+            err = O.error_stats(y.cpu().numpy().reshape(1, -1), ref.reshape(1, -1))
+            assert err["rel_l2"] <= O.north_star_bound(O.Z2Z if double else O.C2C, n0 * n1), (d, err)

@@ -30,6 +30,20 @@ def test_narrow_tiles_below_one_cta_per_sm(n0, n1, code):
     assert "mixed tiles" in _column_pass(n0, n1, code)
 
 
+# 32-byte row segments only below one 64-byte tile per SM, and in single
+# precision only for three stages or more (256 = 16 16, 512 = 8 8 8)
+@pytest.mark.parametrize("n0,n1,code,width", [(256, 512, C2C, 8), (240, 512, C2C, 8), (512, 256, C2C, 4),
+                                              (300, 128, C2C, 4), (256, 256, Z2Z, 2)])
+def test_narrow_tile_width(n0, n1, code, width):
+    assert f"per_cta={width} " in _column_pass(n0, n1, code)
+
+
+# single precision, not a power of two: narrow tiles below half a CTA per SM
+@pytest.mark.parametrize("n1,mixed", [(588, True), (592, False)])
+def test_columns_of_1701(n1, mixed):
+    assert ("mixed tiles" in _column_pass(1701, n1, C2C)) == mixed
+
+
 @pytest.mark.parametrize("n0,n1,code", [(256, 2376, C2C), (512, 2400, C2C), (256, 2376, Z2Z)])
 def test_tile_kernel_from_one_cta_per_sm(n0, n1, code):
     line = _column_pass(n0, n1, code)
