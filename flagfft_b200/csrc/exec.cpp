@@ -609,8 +609,40 @@ class Builder {
     if (fixed && spec.kind == CoreKind::Dit && (io == IoKind::R2C || io == IoKind::C2R))
       return mixed_fits(spec, io, seq) ? seq : std::vector<int>{};
     std::vector<int> r;
-    if (!mixed_chain(L, 0, &r) && !mixed_chain(L, 1, &r)) return {};
-    return mixed_fits(spec, io, r) ? r : std::vector<int>{};
+    const bool small_codelets = mixed_chain(L, 0, &r);
+    if (!small_codelets && !mixed_chain(L, 1, &r)) return {};
+    if (!mixed_fits(spec, io, r)) return {};
+    if (io != IoKind::C2C && spec.kind != CoreKind::Dit && real_convolution_in_place(spec, nbatch * G, small_codelets))
+      return {};
+    return r;
+  }
+
+  // True when the real form of a fused convolution of L points runs on the
+  // in-place tiles, which hold one buffer a transform, rather than on the
+  // mixed-radix ones, which hold two and join the middle stages.  Measured
+  // (us, in place / mixed, R2C or D2Z, `transforms` of them):
+  //   one CTA per SM with two buffers: single precision 8192 points (n = 4079)
+  //   x 1 23.6 / 25.2, x 600 117.8 / 120.2; double 4096 (2003) x 200 21.9 /
+  //   34.4, x 2400 196 / 282, but x 1 18.4 / 18.4 and 4000 (8002) x 1 28.6 /
+  //   24.0;
+  //   single precision, about one wave: 4096 (2003) x 148 15.8 / 17.9, x 296
+  //   17.9 / 18.8, x 350 32.7 / 19.0; 2048 (997) x 148 14.5 / 15.5, x 500 17.4
+  //   / 18.6, x 600 28.7 / 18.7; Rader 4000 (4001) x 148 17.1 / 20.9, x 200
+  //   32.3 / 25.2, but 3000 (6002) x 148 22.3 / 19.6;
+  //   double precision, several waves: 2048 (997) x 444 20.3 / 19.1, x 500 20.3
+  //   / 26.0, x 2400 100.5 / 104.5;
+  //   double precision with a codelet above 10 (one 256-thread CTA per SM):
+  //   Rader 330 (331) x 2400 32.4 / 24.0, x 3200 34.9 / 39.1, x 8192 65.3 /
+  //   91.4; 198 (199) x 8192 58.3 / 42.0.
+  static bool real_convolution_in_place(const CoreSpec &spec, int64_t transforms, bool small_codelets) {
+    const int64_t L = spec.L;
+    const bool bluestein = spec.kind == CoreKind::Bluestein;
+    const bool one_per_sm = kSmSmem / (2 * (size_t)L * sizeof(cpx<T>) + kCtaSmem) < 2;
+    if (sizeof(T) == 4)
+      return one_per_sm || (bluestein && L >= 2048 && transforms * L <= kSMs * 8192) ||
+             (L >= 4000 && transforms <= kSMs);
+    return (one_per_sm && transforms > kSMs) || (bluestein && L >= 2048 && transforms > 3 * kSMs) ||
+           (!small_codelets && L >= 256 && transforms * L >= 1 << 20);
   }
 
   // A transform of the chain fits one CTA and its global runs are long enough.
