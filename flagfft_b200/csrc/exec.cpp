@@ -584,12 +584,17 @@ class Builder {
       int tw = 0, th = 0;
       size_t sm = 0;
       if (fixed && spec.kind == CoreKind::Dit && strided) {
-        // The column kernel keeps every pass that it can copy (buffers off
-        // its rules take the tile kernel).  Against it the narrow tiles were
-        // slower however few its groups: columns of a 2-D C2C, us here and
-        // there with the rows, 1024 x 16 14.2 / 10.6, x 128 13.2 / 8.8, x 512
-        // 15.8 / 12.4, 2048 x 128 11.7 / 9.7; Z2Z 1536 x 16 12.0 / 10.9.
-        if (tcols(spec, io, nbatch, G, ib, ig, ii, ob, og, ok, &th, &sm)) return {};
+        // The column kernel keeps every pass that it can copy.  Against it the
+        // narrow tiles were slower however few its groups: columns of a 2-D
+        // C2C, us here and there with the rows, 1024 x 16 14.2 / 10.6, x 128
+        // 13.2 / 8.8, x 512 15.8 / 12.4, 2048 x 128 11.7 / 9.7; Z2Z 1536 x 16
+        // 12.0 / 10.9.  Buffers off its rules take the tile kernel, from 2048
+        // points on this one: off 16 bytes, us here and there, 2-D 2048 x 2048
+        // 52.5 / 63.2, 2^22 x 1 80.5 / 118, but 1024 x 1024 23.6 / 17.4, 1536 x
+        // 2048 35.9 / 30.9.
+        if (tcols(spec, io, nbatch, G, ib, ig, ii, ob, og, ok, &th, &sm))
+          return sizeof(T) == 4 && L >= 2048 && nbatch <= 65535 && mixed_fits(spec, io, seq, 4) ? seq
+                                                                                               : std::vector<int>{};
         // A tile kernel with fewer CTAs than SMs leaves some idle.  In single
         // precision a sequence with radices other than 2^k gains from the
         // narrow tiles only where it would leave half of them idle
@@ -607,11 +612,11 @@ class Builder {
     // (a half-length real pass of a compile-time sequence keeps it: the real
     // row kernel takes it whenever its rows start on pairs)
     if (fixed && spec.kind == CoreKind::Dit && (io == IoKind::R2C || io == IoKind::C2R))
-      return mixed_fits(spec, io, seq) ? seq : std::vector<int>{};
+      return mixed_fits(spec, io, seq, 1) ? seq : std::vector<int>{};
     std::vector<int> r;
     const bool small_codelets = mixed_chain(L, 0, &r);
     if (!small_codelets && !mixed_chain(L, 1, &r)) return {};
-    if (!mixed_fits(spec, io, r)) return {};
+    if (!mixed_fits(spec, io, r, 1)) return {};
     if (io != IoKind::C2C && spec.kind != CoreKind::Dit && real_convolution_in_place(spec, nbatch * G, small_codelets))
       return {};
     return r;
@@ -645,15 +650,15 @@ class Builder {
            (!small_codelets && L >= 256 && transforms * L >= 1 << 20);
   }
 
-  // A transform of the chain fits one CTA and its global runs are long enough.
-  static bool mixed_fits(const CoreSpec &spec, IoKind io, const std::vector<int> &r) {
+  // W transforms of the chain fit one CTA and its global runs are long enough.
+  static bool mixed_fits(const CoreSpec &spec, IoKind io, const std::vector<int> &r, int W) {
     const int64_t L = spec.L;
     if (r.size() < 2 || (int)r.size() > kMaxStages || L / r.front() < 4 || L / r.back() < 4) return false;
     Core c{};
     c.L = (int)L;
     c.nst = (int)r.size();
     c.radix[0] = r[0];
-    return ((size_t)mixed::slot_len(c, mixed::buffers(c, spec.kind, io)) + 2) * sizeof(cpx<T>) <= 232448;
+    return (size_t)W * ((size_t)mixed::slot_len(c, mixed::buffers(c, spec.kind, io)) + 2) * sizeof(cpx<T>) <= 232448;
   }
 
   // The column kernel takes the pass (tcols.cuh).
@@ -829,6 +834,15 @@ class Builder {
       if (W_overflows(a.W, L, ig, ii) || W_overflows(a.W, L, og, ok))
         throw std::runtime_error("tile extent above 2^31 elements");
       a.tpt = 1;
+      {
+        int th = 0;
+        size_t sm = 0;
+        if (tcols(spec, io, nbatch, G, ib, ig, ii, ob, og, ok, &th, &sm)) {
+          a.tcols = 1;
+          a.tc_threads = th;
+          a.tc_smem = (int)sm;
+        }
+      }
       a.wdiv = make_fastdiv((uint32_t)a.W);
       a.pairs_div = make_fastdiv((uint32_t)(std::max<int64_t>(0, logical_n) / 2 / 2 + 1));
       p->kind = spec.kind;

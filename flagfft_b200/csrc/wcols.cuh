@@ -24,8 +24,9 @@
 //
 // Measured on one B200 against tcols.cuh's kernel: the passes of R2C + C2R
 // 2^24 x 4 (2048 and 4096 points) 1003 -> 821 us with the Hermitian passes,
-// 2-D 4096 x 4096 164 -> 142 us.  A pass moves 3.6 TB/s; a plain copy of the
-// same 32-byte row segments moves 4.3 TB/s, one of 128-byte segments 5.1, so
+// 2-D 4096 x 4096 164 -> 142 us.  A pass moves 3.2 to 3.3 TB/s (537 MB each of
+// the four of 2^24 x 4 in 163 us, the 268 MB of 4096 x 4096 in 85); a plain copy
+// of the same 32-byte row segments moves 4.3, one of 128-byte segments 5.1, so
 // what bounds it is the strided traffic, then the lockstep of one CTA's
 // stages.  Tried and not kept: thread copies (cp.async) instead of TMA, which
 // hold the warps at the load unit at sixteen lines an instruction (2-D 4096 x
@@ -86,7 +87,6 @@ struct alignas(64) Args {
   TileArgs<float> a;
   long long tiles_per_batch;  // ceil(G / W)
   long long total_tiles;      // tiles_per_batch * nbatch
-  int out_aligned;            // adjacent outputs of a column pair may go in one 16-byte store
 };
 
 // W_N^m (conjugated for the inverse) from the two split tables, m < N.
@@ -225,16 +225,14 @@ FFB_HD void write_out(int tid, const typename StageOf<Sh, Sh::Q::n - 1>::Regs &s
   int p, t;
   place<Sh, !OUT_ROWS>(tid, p, t);
   const long long g = g0 + p * 2;
-  if (g >= a.G) return;
-  const bool both = g + 1 < a.G;
+  if (g >= a.G) return;  // (the columns come in pairs)
 #pragma unroll
   for (int u = 0; u < O::U; ++u) {
     if (!O::live(t, u)) continue;
     const int j = t + u * Sh::TPT;  // nb == Ns in the last stage: outputs j + q * nb
     cpx<F2> t0;
     if (a.post_twiddle) {
-      const C32 w0 = split_root(a, (uint32_t)(g * j));
-      const C32 w1 = both ? split_root(a, (uint32_t)((g + 1) * j)) : w0;  // dead columns: no reads past the tables
+      const C32 w0 = split_root(a, (uint32_t)(g * j)), w1 = split_root(a, (uint32_t)((g + 1) * j));
       t0 = mk(F2(w0.x, w1.x), F2(w0.y, w1.y));
     }
     C32 *out = reinterpret_cast<C32 *>(a.out) + b * a.ob + g * a.og + (long long)j * a.ok;
@@ -255,7 +253,7 @@ FFB_HD void write_out(int tid, const typename StageOf<Sh, Sh::Q::n - 1>::Regs &s
       C32 c0, c1;
       v.x.get(c0.x, c1.x);
       v.y.get(c0.y, c1.y);
-      if (!OUT_ROWS && args.out_aligned && both) {
+      if constexpr (!OUT_ROWS) {
 #ifdef __CUDA_ARCH__
         *reinterpret_cast<float4 *>(o) = make_float4(c0.x, c0.y, c1.x, c1.y);
 #else
@@ -264,7 +262,7 @@ FFB_HD void write_out(int tid, const typename StageOf<Sh, Sh::Q::n - 1>::Regs &s
 #endif
       } else {
         o[0] = c0;
-        if (both) o[a.og] = c1;
+        o[a.og] = c1;
       }
     }
   }

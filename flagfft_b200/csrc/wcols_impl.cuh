@@ -28,16 +28,20 @@ inline long long min_tiles() { return kMinTilesPerSm; }  // (so small passes exe
 template <int L, class Sh>
 bool make_args(const TileArgs<float> &a, Args *p, bool *out_rows) {
   if (a.G < Sh::W || a.G >= (1ll << 30) || a.nbatch * (a.G / Sh::W) < min_tiles()) return false;
-  if (a.ig != 1 || a.ii < a.G) return false;
+  if (a.ig != 1 || a.ii < a.G || a.G % 2 != 0) return false;
   *out_rows = a.ok == 1 && a.og >= L;
-  if (!*out_rows && (a.og != 1 || a.ok < a.G)) return false;
+  // (the outputs of a column pair go in one 16-byte store; in two of 8 bytes
+  // the pass lost to the tile kernel: C2C 2^24 x 4 off 16 bytes 2044 us against
+  // 1601, 2^23 x 4 882 against 764)
+  if (!*out_rows && (a.og != 1 || a.ok < a.G || reinterpret_cast<uintptr_t>(a.out) % 16 != 0 || a.ok % 2 != 0 ||
+                     (a.nbatch > 1 && a.ob % 2 != 0)))
+    return false;
   int in_rows = 0;
   if (!tcols::make_view<float, L, Sh::W, Sh::RB>(a.in, a.nbatch, a.G, a.ib, a.ig, a.ii, &p->in_view, &in_rows) || in_rows)
     return false;
   p->a = a;
   p->tiles_per_batch = (a.G + Sh::W - 1) / Sh::W;
   p->total_tiles = p->tiles_per_batch * a.nbatch;
-  p->out_aligned = reinterpret_cast<uintptr_t>(a.out) % 16 == 0 && a.ok % 2 == 0 && (a.nbatch == 1 || a.ob % 2 == 0);
   return true;
 }
 

@@ -22,7 +22,9 @@ def _column_pass(n0, n1, code):
                                         (1024, 64, Z2Z), (1536, 16, Z2Z), (2048, 8, Z2Z)])
 def test_column_kernel_keeps_few_groups(n0, n1, code):
     line = _column_pass(n0, n1, code)
-    assert "tma-columns(" in line and "mixed tiles" not in line, line
+    assert "tma-columns(" in line, line
+    # (the fallback for buffers off 16 bytes)
+    assert ("mixed tiles" in line) == (n0 == 2048 and code == C2C), line
 
 
 @pytest.mark.parametrize("n0,n1,code", [(512, 256, C2C), (256, 512, C2C), (256, 512, Z2Z), (512, 512, Z2Z)])
@@ -50,9 +52,10 @@ def test_tile_kernel_from_one_cta_per_sm(n0, n1, code):
     assert " tiles smem" in line and "mixed" not in line and "tma-columns" not in line, line
 
 
-@pytest.mark.parametrize("n0,n1", [(1024, 20), (2048, 24)])
+@pytest.mark.parametrize("n0,n1", [(1024, 20), (2048, 24), (1024, 66), (2048, 34), (4096, 18)])
 def test_columns_off_16_bytes(n0, n1):
-    """Single-precision columns of a buffer on 8 bytes only: the tile kernel."""
+    """Single-precision columns of a buffer on 8 bytes only: the tile and the
+    mixed-radix kernels, also where an aligned pass takes the wide columns."""
     rng = np.random.default_rng(n0)
     raw = (rng.uniform(-1, 1, n0 * n1 + 4) + 1j * rng.uniform(-1, 1, n0 * n1 + 4)).astype(np.complex64)
     first = 1 if raw.ctypes.data % 16 == 0 else 0
