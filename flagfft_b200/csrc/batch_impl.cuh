@@ -59,8 +59,8 @@ int batch_resident_ctas(int threads, size_t smem) {
   return per_sm * sms;
 }
 #else
-// Sequential host run: the ping-pong bodies with one "thread" per slot
-// (HostX), every transform of a register-column chunk in turn.
+// Sequential host run: the tile bodies with one "thread" (HostX), every
+// transform of a register-column chunk in turn.
 template <typename T>
 cudaError_t launch_batch(const TileArgs<T> *args, const int *kinds, const BatchItem *items, int nitems, int *next,
                          int threads, size_t smem, int, cudaStream_t) {

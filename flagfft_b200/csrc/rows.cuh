@@ -556,12 +556,14 @@ size_t rows_smem(const TileArgs<T> &a) {
 // CTAs' worth of rows per SM instead of one, without spills to speak of.  Its
 // rows each take longer (less of a butterfly's latency is hidden within a
 // thread), so it is for passes whose rows come in several waves: kDensePoints
-// points or more.  Measured (us, 96-128 registers -> 64): C2C 4096 x 4096 56.2
-// -> 49.1, 8192 x 2048 80.2 -> 64.5, Bluestein 4079 x 2000 139 -> 119, 2039 x
-// 4000 94.9 -> 87.6, 509 x 20000 94.8 -> 87.6; but 4096 x 256 5.7 -> 7.0, 8192 x
-// 100 6.0 -> 8.4, 1009 x 1024 12.9 -> 14.5, 509 x 2000 12.1 -> 13.8.  Plain
-// rows of 2048 points or fewer move HBM at its rate either way (1024 x 16384
-// 44.7 -> 44.4), and 1536 loses (8000 rows 36.3 -> 42.1).
+// points or more.  Measured (us, 96-128 registers -> 64) from that line on, C2C
+// 4096 x 1024 17.6 -> 15.8, x 1448 23.1 -> 20.4, x 4096 56.7 -> 48.8; 8192 x 512
+// 24.5 -> 20.8, x 2048 79.8 -> 64.1; Bluestein 509 x 4096 23.2 -> 21.4, 1009 x
+// 2048 23.8 -> 22.9, 2039 x 1024 29.6 -> 26.6, 4079 x 512 41.1 -> 37.2, x 2048
+// 140 -> 118; but below it 4096 x 256 5.7 -> 7.0, 8192 x 100 6.0 -> 8.4, 1009 x
+// 1024 12.9 -> 14.5, 509 x 2000 12.1 -> 13.8.  Plain rows of 2048 points or
+// fewer move HBM at its rate either way (1024 x 16384 44.7 -> 44.4), and 1536
+// loses (8000 rows 36.3 -> 42.1).
 constexpr long long kDensePoints = 1ll << 22;
 template <typename T, int KIND, int L>
 constexpr bool rows_dense() {

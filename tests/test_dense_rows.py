@@ -1,5 +1,6 @@
-"""The 64-register row kernels (csrc/rows.cuh rows_dense, csrc/rrows.cuh): the
-smallest pass that takes them and one row fewer, a part tile, both directions.
+"""The 64-register row kernels (csrc/rows.cuh rows_dense, csrc/rrows.cuh): one
+row more and one fewer than the smallest pass that takes them, a part tile,
+both directions.
 Bounds: the parity bar 5e-7 log2 N against an FP64 transform."""
 import math
 

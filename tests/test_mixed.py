@@ -58,7 +58,7 @@ def test_emulated_strided(n0, n1):
 
 @pytest.mark.parametrize("double", [False, True])
 def test_emulated_unaligned_reals(double):
-    """Real rows of odd distance from an address off a pair: the scalar loads."""
+    """Real rows from an address off a pair: the scalar loads."""
     n, batch, dist = 250, 5, 250
     rng = np.random.default_rng(5)
     t = np.float64 if double else np.float32

@@ -1,6 +1,6 @@
 """The wide column kernel (csrc/wcols.cuh): every sequence, column and row
-outputs with the four-step twiddle, last tiles with one live column of a pair
-and with dead pairs.  Bounds: the parity bar 5e-7 log2 N against an FP64
+outputs with the four-step twiddle, last tiles with dead column pairs (columns
+come in pairs: a tensor copy wants an even row length).  Bounds: the parity bar 5e-7 log2 N against an FP64
 transform.  The CPU tests run the kernel body in host emulation, which takes
 passes of four tiles or more."""
 import math
