@@ -589,12 +589,13 @@ class Builder {
         // C2C, us here and there with the rows, 1024 x 16 14.2 / 10.6, x 128
         // 13.2 / 8.8, x 512 15.8 / 12.4, 2048 x 128 11.7 / 9.7; Z2Z 1536 x 16
         // 12.0 / 10.9.  Buffers off its rules take the tile kernel, from 2048
-        // points on this one: off 16 bytes, us here and there, 2-D 2048 x 2048
-        // 52.5 / 63.2, 2^22 x 1 80.5 / 118, but 1024 x 1024 23.6 / 17.4, 1536 x
-        // 2048 35.9 / 30.9.
+        // points and columns on this one: off 16 bytes, us here and there, 2-D
+        // 2048 x 2048 52.5 / 63.2, 2^22 x 1 80.5 / 118, but 1024 x 1024 23.6 /
+        // 17.4, 1536 x 2048 35.9 / 30.9, 2^21 x 4 156 / 135.
         if (tcols(spec, io, nbatch, G, ib, ig, ii, ob, og, ok, &th, &sm))
-          return sizeof(T) == 4 && L >= 2048 && nbatch <= 65535 && mixed_fits(spec, io, seq, 4) ? seq
-                                                                                               : std::vector<int>{};
+          return sizeof(T) == 4 && L >= 2048 && G >= 2048 && nbatch <= 65535 && mixed_fits(spec, io, seq, 4)
+                     ? seq
+                     : std::vector<int>{};
         // A tile kernel with fewer CTAs than SMs leaves some idle.  In single
         // precision a sequence with radices other than 2^k gains from the
         // narrow tiles only where it would leave half of them idle
@@ -717,17 +718,31 @@ class Builder {
     const int64_t wide = sizeof(T) == 4 ? 8 : 4;
     if (strided) {
       const bool halve = a.nbatch * a.G / wide < kSMs && (sizeof(T) == 8 || a.core.nst > 2);
-      for (least = std::min<int64_t>(halve ? wide / 2 : wide, a.G);
-           least > 1 && mixed::smem_bytes(a, kind, io, (int)least) > 232448; --least) {
+      // a long convolution's time is its stages, not its rows: no wider than
+      // leaves every SM a tile, or one SM three (us, before / so: C2C 3027 x 60
+      // 25.4 / 18.3, 2018 x 1 18.7 / 17.3, 12108 x 173 128 / 75.5; but of 66
+      // points 134 x 1 10.0 / 11.1)
+      auto too_wide = [&](int64_t W) {
+        const size_t smem = mixed::smem_bytes(a, kind, io, (int)W);
+        return smem > 232448 || (kind != CoreKind::Dit && a.core.L >= 2048 &&
+                                 (a.nbatch * ((a.G + W - 1) / W) < kSMs || 3 * (smem + kCtaSmem) > kSmSmem));
+      };
+      for (least = std::min<int64_t>(halve ? wide / 2 : wide, a.G); least > 1 && too_wide(least); --least) {
       }
     }
+    // (one warp where the widest tile's widest stage leaves some of two idle:
+    // Z2Z 134 x 15650 163 -> 114.5 us, 201 x 10433 124 -> 95.5)
+    const bool short_tile = most * (a.core.L / *std::min_element(a.core.radix, a.core.radix + a.core.nst)) < 64;
     double best = 1e300;
-    for (int NT = 64; NT <= mixed::kMaxThreads; NT += 32)
+    for (int NT = short_tile ? 32 : 64; NT <= mixed::kMaxThreads; NT += 32)
       for (int64_t W = least; W <= most; ++W) {
         const size_t smem = mixed::smem_bytes(a, kind, io, (int)W);
         if (smem > 232448) break;
-        const int64_t per_sm =
-            std::min<int64_t>({65536 / (regs * NT), (int64_t)(kSmSmem / (smem + kCtaSmem)), 2048 / NT, 32});
+        // (a tile that fits a CTA counts one per SM, however full; with the
+        // exact count, 233472 bytes, the shapes it moves lose: C2C 2000 x 1024
+        // 17.7 -> 22.3 us, 2-D 2000 x 2000 68 -> 74)
+        const int64_t per_sm = std::min<int64_t>(
+            {65536 / (regs * NT), std::max<int64_t>(1, (int64_t)(232448 / (smem + kCtaSmem))), 2048 / NT, 32});
         if (per_sm < 1) continue;
         const int64_t tiles = a.nbatch * ((a.G + W - 1) / W);
         double issue = 0, latency = 2000;

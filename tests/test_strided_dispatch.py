@@ -24,7 +24,13 @@ def test_column_kernel_keeps_few_groups(n0, n1, code):
     line = _column_pass(n0, n1, code)
     assert "tma-columns(" in line, line
     # (the fallback for buffers off 16 bytes)
-    assert ("mixed tiles" in line) == (n0 == 2048 and code == C2C), line
+    assert "mixed tiles" not in line, line
+
+
+@pytest.mark.parametrize("n0,n1,mixed", [(2048, 2048, True), (2048, 2040, False), (1536, 2048, False)])
+def test_fallback_off_16_bytes(n0, n1, mixed):
+    line = _column_pass(n0, n1, C2C)
+    assert "tma-columns(" in line and ("mixed tiles" in line) == mixed, line
 
 
 @pytest.mark.parametrize("n0,n1,code", [(512, 256, C2C), (256, 512, C2C), (256, 512, Z2Z), (512, 512, Z2Z)])
@@ -67,3 +73,26 @@ def test_columns_off_16_bytes(n0, n1):
     H.lib().flagfftDestroy(plan)
     ref = np.fft.fft2(x.reshape(n0, n1).astype(np.complex128)).ravel()
     assert np.linalg.norm(out - ref) <= 5e-7 * np.log2(n0 * n1) * np.linalg.norm(ref)
+
+
+# a prime times a small factor: the convolutions of the second pass, whose
+# outputs are strided, take no more of a tile than leaves every SM one, or an
+# SM three; a tile of a few butterflies one warp
+@pytest.mark.parametrize("n,batch,code,shape", [(3027, 60, C2C, "per_cta=1 threads=256 "),
+                                                (12108, 173, C2C, "per_cta=2 threads=256 "),
+                                                (134, 15650, Z2Z, "per_cta=2 threads=32 ")])
+def test_strided_convolution_tiles(n, batch, code, shape):
+    plan = H.plan1d(n, code, batch)
+    text = H.describe(plan).split("-- Forward execution --")[-1].split("-- Inverse execution --")[0]
+    H.lib().flagfftDestroy(plan)
+    line = [ln for ln in text.splitlines() if ln.strip().startswith("pass ")][1]
+    assert shape in line and "mixed tiles" in line, line
+
+
+@pytest.mark.parametrize("n,batch,double", [(2018, 2, False), (3027, 60, False), (134, 40, True), (201, 3, True)])
+def test_strided_convolution_values(n, batch, double):
+    rng = np.random.default_rng(n)
+    x = rng.uniform(-1, 1, (batch, n)) + 1j * rng.uniform(-1, 1, (batch, n))
+    bound = (1e-15 if double else 5e-7) * np.log2(n)
+    for d, ref in ((-1, np.fft.fft(x)), (1, np.fft.ifft(x, norm="forward"))):
+        assert np.linalg.norm(H.c2c(x, d, double) - ref) <= bound * np.linalg.norm(ref)
