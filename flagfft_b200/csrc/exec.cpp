@@ -406,7 +406,7 @@ bool own_four_step(int64_t n, int64_t maxL, int64_t *n1_out, std::vector<int> *r
 }
 }  // namespace
 
-static Core make_dit_core(int64_t L, const std::vector<int> &r) {
+static Core make_dit_core(int64_t L, const std::vector<int> &r, bool in_place) {
   if ((int)r.size() > kMaxStages) throw std::runtime_error("too many radix stages");
   Core c{};
   c.L = (int)L;
@@ -416,8 +416,7 @@ static Core make_dit_core(int64_t L, const std::vector<int> &r) {
     c.radix[s] = r[s];
     c.span[s] = (int)span;
     c.sdiv[s] = make_fastdiv((uint32_t)span);
-    c.rdiv[s] = make_fastdiv((uint32_t)r[s]);
-    c.bdiv[s] = make_fastdiv((uint32_t)(L / r[s]));
+    c.rdiv[s] = make_fastdiv((uint32_t)(in_place ? r[s] : L / r[s]));
     span *= r[s];
   }
   if (span != L) throw std::runtime_error("radices do not multiply to the core length");
@@ -435,7 +434,6 @@ static Core make_dif_core(int64_t L, const std::vector<int> &r) {
     c.span[s] = (int)span;
     c.sdiv[s] = make_fastdiv((uint32_t)(span / r[s]));
     c.rdiv[s] = make_fastdiv((uint32_t)r[s]);
-    c.bdiv[s] = make_fastdiv((uint32_t)(L / r[s]));
     span /= r[s];
   }
   if (span != 1) throw std::runtime_error("radices do not multiply to the core length");
@@ -809,12 +807,12 @@ class Builder {
     std::vector<int> radices = mixed_r.empty() ? spec.radices : mixed_r;
     if (a.pp) std::sort(radices.rbegin(), radices.rend());
     if (spec.kind == CoreKind::Dit) {
-      a.core = make_dit_core(L, radices);
+      a.core = make_dit_core(L, radices, !a.pp);
     } else {
-      a.core = a.pp ? make_dit_core(L, radices) : make_dif_core(L, radices);
+      a.core = a.pp ? make_dit_core(L, radices, false) : make_dif_core(L, radices);
       std::vector<int> rev(radices.rbegin(), radices.rend());
       const bool row_kernel = a.pp && mixed_r.empty() && (!t_no_one_pass || a.rows_only);
-      a.core2 = make_dit_core(L, row_kernel ? radices : rev);
+      a.core2 = make_dit_core(L, row_kernel ? radices : rev, !a.pp);
       if (spec.kind != CoreKind::Conv) fill_convolution(a, spec, inverse);  // Conv: caller supplies the kernel
     }
     // one-codelet transforms lying side by side in memory on both sides run
@@ -1386,7 +1384,7 @@ void lower_c2c(Builder<T> &bld, Program &prog, const NodePtr &root, bool inverse
       a.chirp = bld.table_chirp(n, inverse);
       a.kern = bld.table_bluestein_rows(n, row_radices, n1, n2, inverse, true);
       a.kern_stride = n2;
-      a.core2 = make_dit_core(n2, std::vector<int>(row_radices.rbegin(), row_radices.rend()));
+      a.core2 = make_dit_core(n2, std::vector<int>(row_radices.rbegin(), row_radices.rend()), false);
       a.tw2 = bld.table_stage_twiddles(a.core2, false, true);
       bld.set_post_twiddle(a, M);
       p->smem = blue4_smem((int)n1, (int)n2, sizeof(cpx<T>), pair);

@@ -306,7 +306,7 @@ FFB_HD void run_chain(const Tile<T> &t, const Core &c, const cpx<T> *__restrict_
       j = (int)fdiv((uint32_t)e, a.wdiv);
       w = e - j * W;
     } else {
-      w = (int)fdiv((uint32_t)e, c.bdiv[s]);
+      w = (int)fdiv((uint32_t)e, c.rdiv[s]);
       j = e - w * nb;
     }
   };
