@@ -30,12 +30,15 @@ bool make_args(const TileArgs<float> &a, Args *p, bool *out_rows) {
   if (a.G < Sh::W || a.G >= (1ll << 30) || a.nbatch * (a.G / Sh::W) < min_tiles()) return false;
   if (a.ig != 1 || a.ii < a.G || a.G % 2 != 0) return false;
   *out_rows = a.ok == 1 && a.og >= L;
-  // (the outputs of a column pair go in one 16-byte store; in two of 8 bytes
-  // the pass lost to the tile kernel: C2C 2^24 x 4 off 16 bytes 2044 us against
-  // 1601, 2^23 x 4 882 against 764)
-  if (!*out_rows && (a.og != 1 || a.ok < a.G || reinterpret_cast<uintptr_t>(a.out) % 16 != 0 || a.ok % 2 != 0 ||
-                     (a.nbatch > 1 && a.ob % 2 != 0)))
-    return false;
+  // rows of 1024 points: the column kernel writes them faster (C2C 2^20 x 16 140
+  // us here, 132 there, R2C 2^21 x 16 197 / 187; 1536 x 2048 points x 8 210 / 224,
+  // 2^22 x 8 262 / 290)
+  if (*out_rows && L < 1536) return false;
+  if (!*out_rows && (a.og != 1 || a.ok < a.G)) return false;
+  // outputs off 16 bytes, two stores for one: the tile kernel is faster (C2C
+  // 2^24 x 4 2044 us here, 1601 there, 2^23 x 4 882 / 764)
+  p->out_aligned = reinterpret_cast<uintptr_t>(a.out) % 16 == 0 && a.ok % 2 == 0 && (a.nbatch == 1 || a.ob % 2 == 0);
+  if (!*out_rows && !p->out_aligned) return false;
   int in_rows = 0;
   if (!tcols::make_view<float, L, Sh::W, Sh::RB>(a.in, a.nbatch, a.G, a.ib, a.ig, a.ii, &p->in_view, &in_rows) || in_rows)
     return false;
@@ -62,10 +65,10 @@ cudaError_t launch_seq(const TileArgs<float> &a, cudaStream_t s) {
     if ((e = set_smem_limit_once<k_wcols<INV, L, OR, Rs...>>((int)Sh::smem)) != cudaSuccess) return e;       \
     return launch_pdl(k, dim3((unsigned)ctas), dim3(Sh::NT), Sh::smem, s, p);                                \
   }
-  if (out_rows)
-    FFB_WCOLS_GO(true)
-  else
-    FFB_WCOLS_GO(false)
+  if constexpr (L >= 1536) {
+    if (out_rows) FFB_WCOLS_GO(true)
+  }
+  FFB_WCOLS_GO(false)
 #undef FFB_WCOLS_GO
 }
 

@@ -36,3 +36,10 @@ def test_real_rows_shape():
 def test_columns(n0, n1, code, wide):
     line = _passes(H.plan2d(n0, n1, code))[1]
     assert ("wide-tma-columns" in line) == wide and "tma-columns(threads=" in line, line
+
+
+def test_rows_of_1024_points_from_the_column_kernel():
+    """A four-step's first pass of 1024 points writes rows: not the wide form."""
+    first, second = _passes(H.plan1d(1 << 20, C2C, 4))
+    assert " tma-columns(" in first and "+twiddle" in first and "wide" not in first, first
+    assert "wide-tma-columns(" in second, second
