@@ -728,9 +728,12 @@ class Builder {
       for (least = std::min<int64_t>(halve ? wide / 2 : wide, a.G); least > 1 && too_wide(least); --least) {
       }
     }
-    // (one warp where the widest tile's widest stage leaves some of two idle:
-    // Z2Z 134 x 15650 163 -> 114.5 us, 201 x 10433 124 -> 95.5)
-    const bool short_tile = most * (a.core.L / *std::min_element(a.core.radix, a.core.radix + a.core.nst)) < 64;
+    // One warp a CTA where the widest tile's widest stage leaves some of two idle
+    // and registers, not tiles, bound the SM (sixteen tiles each and more): Z2Z
+    // 134 x 15650 163 -> 114.5 us, 201 x 10433 124 -> 95.5.
+    const bool short_tile =
+        most * (a.core.L / *std::min_element(a.core.radix, a.core.radix + a.core.nst)) < 64 &&
+        a.nbatch * ((a.G + most - 1) / most) >= 16 * kSMs;
     double best = 1e300;
     for (int NT = short_tile ? 32 : 64; NT <= mixed::kMaxThreads; NT += 32)
       for (int64_t W = least; W <= most; ++W) {
